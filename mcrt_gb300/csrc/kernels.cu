@@ -14,8 +14,9 @@
 //                        material in shared memory; continuing paths, ended paths and
 //                        next-event rays are appended to SoA queues by warp ballot /
 //                        warp prefix sum + one atomic per warp
-//     k_connect          next-event rays: any hit (environment) or bounded closest hit
-//                        (area lights, which must hit the sampled emitter), MIS-weighted
+//     k_shadow           next-event rays to the environment: any hit
+//     k_connect          next-event rays to area lights: bounded closest hit (which must be
+//                        the sampled emitter), MIS-weighted
 //   k_adjoint            path-replay adjoint (one thread per path, replayed from its seed)
 #include <cuda_runtime.h>
 
@@ -781,11 +782,20 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                     atomicOr(a.err, kErrQueue);
                     break;
                 }
-                // .w: where a closest-hit ray stops at a nearer hit (tmin is kEpsRay for all)
-                a.so[qsel][idx] = make_float4(phit.x, phit.y, phit.z, nee[r].tterm);
-                a.sd[qsel][idx] = make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, nee[r].tmax);
-                a.sv[qsel][idx] = nee[r].val;
-                a.sm[qsel][idx] = make_int4(dest + r, nee[r].type | (nee[r].light << 2), pixel, job);
+                if (qsel == 0)
+                {
+                    a.so[0][idx] = make_float4(phit.x, phit.y, phit.z, __int_as_float(dest + r));
+                    a.sd[0][idx] = make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, __int_as_float(job));
+                    a.nev[pn][dest + r] = nee[r].val;
+                }
+                else
+                {
+                    // .w: where a closest-hit ray stops at a nearer hit (tmin is kEpsRay for all)
+                    a.so[1][idx] = make_float4(phit.x, phit.y, phit.z, nee[r].tterm);
+                    a.sd[1][idx] = make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, nee[r].tmax);
+                    a.sv[idx] = nee[r].val;
+                    a.sm[idx] = make_int4(dest + r, nee[r].type | (nee[r].light << 2), pixel, job);
+                }
             }
         }
         pos += 128;
@@ -797,16 +807,16 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
 // Adjoint (ADJ): the emission derivative of each next-event contribution (the
 // coefficient of the reached emitter's E)
 template <bool ADJ>
-__device__ __forceinline__ void connect_result(const WaveArgs& a, const Grads& G, int p, int q, int k, bool hit,
+__device__ __forceinline__ void connect_result(const WaveArgs& a, const Grads& G, int p, int k, float3 d, bool hit,
                                                const Hit& h)
 {
-    const float4     d = a.sd[q][k], v = a.sv[q][k];
-    const int4       m = a.sm[q][k];
+    const float4     v = a.sv[k];
+    const int4       m = a.sm[k];
     const JobGPU&    J = a.jobs[m.w];
     const SceneView& S = J.scene;
     float3           coef;
     int              emat;
-    float3           add = nee_contribution(S, m.y & 3, m.y >> 2, v, xyz(d), hit, h, coef, emat);
+    float3           add = nee_contribution(S, m.y & 3, m.y >> 2, v, d, hit, h, coef, emat);
     a.nev[p ^ 1][m.x] = make_float4(add.x, add.y, add.z, 0.f);
     if (ADJ && emat >= 0)
     {
@@ -815,33 +825,55 @@ __device__ __forceinline__ void connect_result(const WaveArgs& a, const Grads& G
     }
 }
 
-// Q = 0: the any-hit queue (rays to the environment); Q = 1: the bounded closest-hit
-// queue (rays to area lights).  One kernel per queue: the any-hit build needs no
-// closest-hit state, so it fits 56 registers without spills (both in one kernel spilled
-// 80 B; next-event stage 37.8 -> 37.5 ms per cfg1 frame) and runs capped at 40 registers
-// for 12 blocks per SM (kAnyHitMinBlocks; its adjoint build at 10, kAnyHitMinBlocksAdj).
-template <int STACK, bool COUNT, int MINB, bool ADJ, int Q, bool REFM = true>
-__global__ void __launch_bounds__(kTraceBlock,
-                                  (Q == 0 && MINB > 1) ? (ADJ ? kAnyHitMinBlocksAdj : kAnyHitMinBlocks) : MINB)
-    k_connect(WaveArgs a, int p)
+// The any-hit queue (next-event rays to the environment).  k_shade has written the value an
+// unoccluded ray adds to the slot its path will read; an occluded ray clears the slot.  So a
+// queue entry is a ray with its slot and job, 32 B instead of 64, and a ray that gets through
+// writes nothing; with the value and the kinds of result out of the kernel it holds fewer
+// registers beside the traversal's (no spills at 48; 12 blocks per SM as before).  Adjoint
+// and forward run the same kernel: an environment ray has no emission derivative.
+template <int STACK, bool COUNT, int MINB, bool REFM = true>
+__global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kAnyHitMinBlocks : MINB) k_shadow(WaveArgs a, int p)
+{
+    __shared__ int stack[STACK * kTraceBlock];
+    int*           st = stack + threadIdx.x;
+    TraceCount     cnt = {0u, 0u};
+    const int      n = min(a.ctrl->scount[0], static_cast<int>(a.shadow_cap));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
+    for (QueueWalk w(&a.ctrl->fetch[1], n, a.batch_fetch != 0); w.valid(); w.next())
+    {
+        const int k = w.i;
+        if (k >= n) continue;
+        const float4  o = a.so[0][k], d = a.sd[0][k];
+        const JobGPU& J = a.jobs[__float_as_int(d.w)];
+        Hit           h;
+        if (trace_ray<true, STACK, COUNT, REFM>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay,
+                                                __int_as_float(0x7f800000), st, kTraceBlock, h, a.err, &cnt))
+            a.nev[p ^ 1][__float_as_int(o.w)] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (COUNT) flush_count(a.stats, 4, cnt);
+}
+
+// the bounded closest-hit queue (next-event rays to area lights)
+template <int STACK, bool COUNT, int MINB, bool ADJ, bool REFM = true>
+__global__ void __launch_bounds__(kTraceBlock, MINB) k_connect(WaveArgs a, int p)
 {
     extern __shared__ float sgrad[];
     __shared__ int stack[STACK * kTraceBlock];
     const Grads    G = grads_begin<ADJ, GRAD_EMISSION>(a, sgrad);
     int*           st = stack + threadIdx.x;
     TraceCount     cnt = {0u, 0u};
-    const int      n = min(a.ctrl->scount[Q], static_cast<int>(a.shadow_cap));
+    const int      n = min(a.ctrl->scount[1], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
-    for (QueueWalk w(&a.ctrl->fetch[1 + Q], n, a.batch_fetch != 0); w.valid(); w.next())
+    for (QueueWalk w(&a.ctrl->fetch[2], n, a.batch_fetch != 0); w.valid(); w.next())
     {
         const int k = w.i;
         if (k >= n) continue;
-        float4        o = a.so[Q][k], d = a.sd[Q][k];
-        const JobGPU& J = a.jobs[a.sm[Q][k].w];
+        const float4  o = a.so[1][k], d = a.sd[1][k];
+        const JobGPU& J = a.jobs[a.sm[k].w];
         Hit           h;
-        bool hit = trace_ray<Q == 0, STACK, COUNT, REFM, Q == 1>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay, d.w,
-                                                                 st, kTraceBlock, h, a.err, &cnt, o.w);
-        connect_result<ADJ>(a, G, p, Q, k, hit, h);
+        bool hit = trace_ray<false, STACK, COUNT, REFM, true>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay, d.w, st,
+                                                              kTraceBlock, h, a.err, &cnt, o.w);
+        connect_result<ADJ>(a, G, p, k, xyz(d), hit, h);
     }
     if (COUNT) flush_count(a.stats, 4, cnt);
     grads_end<ADJ, GRAD_EMISSION>(a, sgrad);
@@ -1448,9 +1480,9 @@ void enqueue_iter(const WaveArgs& a, int p, const LaunchShape& ls, cudaStream_t 
         k_shade<ADJ, 3><<<ls.grid_shade, 128, ds, st>>>(a, p);
     end();
     beg(3);
-    k_connect<STACK, COUNT, MINB, ADJ, 0, REFM><<<ls.grid_any, kTraceBlock, dc, st>>>(a, p);
-    // closest-hit next-event rays exist only where a job has area lights
-    if (ls.lights & 2) k_connect<STACK, COUNT, MINB, ADJ, 1, REFM><<<ls.grid_connect, kTraceBlock, dc, st>>>(a, p);
+    // each kind of next-event ray exists only where a job has that kind of light
+    if (ls.lights & 1) k_shadow<STACK, COUNT, MINB, REFM><<<ls.grid_any, kTraceBlock, 0, st>>>(a, p);
+    if (ls.lights & 2) k_connect<STACK, COUNT, MINB, ADJ, REFM><<<ls.grid_connect, kTraceBlock, dc, st>>>(a, p);
     end();
 }
 
@@ -1492,7 +1524,7 @@ struct RunResult
     int64_t     launches = 0;
     int64_t     extend_launches = 0;
     int64_t     table_bytes = 0;  // host -> device besides the job table
-    int         iter_launches = 6;  // launches per iteration (5 without area lights)
+    int         iter_launches = 6;  // launches per iteration (5 with one kind of light)
     int64_t     poll_bytes = 0;   // device -> host completion polls
 };
 
@@ -1843,15 +1875,14 @@ int adjoint_launch_shape(const WaveArgs& a, LaunchShape& ls)
     CK(cudaFuncSetAttribute(k_shade<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ds));
     CK(cudaFuncSetAttribute(k_shade<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ds));
     constexpr int B = kTraceMinBlocks;
-    CK(cudaFuncSetAttribute(k_connect<STACK, false, B, true, 0, REFM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dc));
-    CK(cudaFuncSetAttribute(k_connect<STACK, false, B, true, 1, REFM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dc));
+    CK(cudaFuncSetAttribute(k_connect<STACK, false, B, true, REFM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dc));
     const int sms = num_sms();
     int       occ_e = 0, occ_s = 0, occ_a = 0, occ_c = 0, occ_r = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_e, k_extend<STACK, false, B, REFM>, kTraceBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_shade<true, 3>, 128, ds);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_regen<true>, 128, dr);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_connect<STACK, false, B, true, 0, REFM>, kTraceBlock, dc);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k_connect<STACK, false, B, true, 1, REFM>, kTraceBlock, dc);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_shadow<STACK, false, B, REFM>, kTraceBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k_connect<STACK, false, B, true, REFM>, kTraceBlock, dc);
     ls.grid_trace = sms * std::max(occ_e, 1);
     ls.grid_any = sms * std::max(occ_a, 1);
     ls.grid_connect = sms * std::max(occ_c, 1);
@@ -1930,7 +1961,7 @@ int adjoint_stream(Workspace& w, const std::vector<JobGPU>& jobs, int64_t total,
     if (rc) return rc;
     ls.fast_only = fast_only;
     ls.lights = lights == 0 ? 3 : lights;
-    run.iter_launches = (ls.lights & 2) ? 6 : 5;
+    run.iter_launches = 4 + (ls.lights & 1) + (ls.lights >> 1);
     auto iter = [&](cudaStream_t s2, int p, StageTimer*) {
         if (stack32)
             fast_only ? enqueue_adjoint_iter<kSmallStack, false>(a, p, ls, s2)
@@ -2035,7 +2066,7 @@ int render_jobs(int num_jobs, mcrt_scene* const* scenes, const mcrt_camera* cams
     w.args.batch_fetch = (vb & MCRT_VARIANT_GRIDSTRIDE) ? 0 : 1;
     StageTimer  timer;
     RunResult   run;
-    run.iter_launches = (lsv.lights & 2) ? 6 : 5;
+    run.iter_launches = 4 + (lsv.lights & 1) + (lsv.lights >> 1);
     int         rc = p0.schedule == MCRT_SCHEDULE_WAVES
                          ? run_waves(w, jobs, pix_spp, total, max_depth, p0.path_chunk, stack32, regcap, count, stages,
                                      graph, lsv, st, timer, run)
@@ -2101,8 +2132,9 @@ size_t queue_bytes(int64_t capacity)
 {
     const size_t C = static_cast<size_t>(capacity);
     // by parity: qo, qd, qthr, qrad (64 B) + qrng 8 + drad, dmeta 32 + nev 128; hits 16;
-    // next-event queues: 2 x 2C x (so, sd, sv, sm) 64 B; 256-B alignment of 31 sub-arrays
-    return 2 * C * (64 + 8 + 32 + 128) + C * 16 + 2 * (2 * C) * 64 + 256 * 32;
+    // next-event queues: 2C x (so, sd) 32 B any-hit, 2C x (so, sd, sv, sm) 64 B closest-hit;
+    // 256-B alignment of 23 sub-arrays
+    return 2 * C * (64 + 8 + 32 + 128) + C * 16 + 2 * C * (32 + 64) + 256 * 32;
 }
 
 void carve_queues(WaveArgs& a, void* base, int64_t capacity)
@@ -2125,9 +2157,9 @@ void carve_queues(WaveArgs& a, void* base, int64_t capacity)
     {
         a.so[k] = static_cast<float4*>(c.take(16 * S));
         a.sd[k] = static_cast<float4*>(c.take(16 * S));
-        a.sv[k] = static_cast<float4*>(c.take(16 * S));
-        a.sm[k] = static_cast<int4*>(c.take(16 * S));
     }
+    a.sv = static_cast<float4*>(c.take(16 * S));
+    a.sm = static_cast<int4*>(c.take(16 * S));
     a.capacity = C;
     a.shadow_cap = S;
 }
@@ -2165,8 +2197,7 @@ LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only)
     if (!fast_only)  // the general build (see with_variant)
     {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_extend<kStack, false, 1, true>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_connect<kStack, false, 1, false, 0, true>, kTraceBlock,
-                                                      0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_shadow<kStack, false, 1, true>, kTraceBlock, 0);
     }
     else if (stack32)
     {
@@ -2175,7 +2206,7 @@ LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only)
             kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &occ_a,
-            regcap ? k_connect<kSmallStack, false, B, false, 0, false> : k_connect<kSmallStack, false, 1, false, 0, false>,
+            regcap ? k_shadow<kSmallStack, false, B, false> : k_shadow<kSmallStack, false, 1, false>,
             kTraceBlock, 0);
     }
     else
@@ -2184,7 +2215,7 @@ LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only)
             &occ_t, regcap ? k_extend<kStack, false, B, false> : k_extend<kStack, false, 1, false>, kTraceBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &occ_a,
-            regcap ? k_connect<kStack, false, B, false, 0, false> : k_connect<kStack, false, 1, false, 0, false>,
+            regcap ? k_shadow<kStack, false, B, false> : k_shadow<kStack, false, 1, false>,
             kTraceBlock, 0);
     }
     ls.fast_only = fast_only;

@@ -41,7 +41,7 @@ constexpr int64_t kNoAllocWaves = 65536;  // waves per render
 constexpr size_t  kHeaderBytes = 4096;    // Ctrl, stats, error word, one JobGPU
 constexpr size_t  kChunkBytes = sizeof(int64_t) * (kNoAllocWaves + 1);
 // queue_bytes(kNoAllocPaths) and ring_bytes(kNoAllocPaths), rounded up; checked at set-up
-constexpr size_t kQueueBytes = (static_cast<size_t>(kNoAllocPaths) * 736 + 256 * 32 + 255) & ~size_t(255);
+constexpr size_t kQueueBytes = (static_cast<size_t>(kNoAllocPaths) * 672 + 256 * 32 + 255) & ~size_t(255);
 constexpr size_t kRingBytes = (static_cast<size_t>(kNoAllocPaths) * 20 + 512 + 255) & ~size_t(255);
 constexpr size_t kNoAllocScratchBytes = kHeaderBytes + kChunkBytes + kQueueBytes + kRingBytes;
 

@@ -15,8 +15,9 @@
 //   k_extend      closest hit of every ray of queue p
 //   k_shade       one vertex per ray: continuing paths to queue p ^ 1, ended paths to
 //                 the finished list p ^ 1, next-event rays to the next-event queues
-//   k_connect     trace the next-event rays; each result goes to the slot its path
-//                 will read next (queue p ^ 1 position or finished-list position)
+//   k_shadow, k_connect   trace the next-event rays (environment, area lights); each result
+//                 goes to the slot its path will read next (queue p ^ 1 position or
+//                 finished-list position)
 #pragma once
 #include <cuda_runtime.h>
 
@@ -43,12 +44,11 @@ constexpr int kTraceMinBlocks = MCRT_TRACE_MIN_BLOCKS;
 // The any-hit next-event kernel under MCRT_VARIANT_REGCAP: 40 registers, 12 blocks per SM
 // (40 B of spills).  Next-event stage per cfg1 frame: 10 blocks (48 registers, no spills)
 // 33.96 ms, 12 blocks 32.53 (an earlier build, with tmin read from the queue and more
-// spills: 9 blocks 37.5, 10 blocks 36.5, 12 blocks 38.8).  Its adjoint build keeps 10.
+// spills: 9 blocks 37.5, 10 blocks 36.5, 12 blocks 38.8).
 #ifndef MCRT_ANYHIT_MIN_BLOCKS
 #define MCRT_ANYHIT_MIN_BLOCKS 12
 #endif
 constexpr int kAnyHitMinBlocks = MCRT_ANYHIT_MIN_BLOCKS;
-constexpr int kAnyHitMinBlocksAdj = 10;
 constexpr int kMaxDepth = 62;
 constexpr int64_t kMaxQueue = int64_t(1) << 27;     // rays per queue (result indices stay in int)
 // Streaming schedule default: 64 M rays (49 GB of queues).  Per cfg1 frame (67 M paths):
@@ -67,7 +67,7 @@ struct Ctrl
     int                new_base;   // this iteration's admitted paths: first queue position
     int                new_count;  //   and how many
     int                chunk;      // wave schedule: index of the current wave
-    int                fetch[3];   // rays taken so far by this iteration's k_extend, k_connect<0>, k_connect<1>
+    int                fetch[3];   // rays taken so far by this iteration's k_extend, k_shadow, k_connect
     unsigned long long next;      // index of the next path to admit
     unsigned long long limit;     // admission limit (exclusive)
     unsigned long long new_g;     // index of the first path admitted this iteration
@@ -97,13 +97,15 @@ struct WaveArgs
     // next-event results by parity: [4 i + s] for queue position i, [4 capacity + 4 j + s]
     // for finished-list position j
     float4* nev[2];
-    // next-event queues: [0] any-hit, [1] closest-hit; origin + stop distance (so.w: a
-    // closest-hit ray stops at a nearer hit, emitter_span), direction + tmax, value,
-    // meta = {result index, type | light << 2, pixel, job}; tmin is kEpsRay for all
+    // next-event queues; tmin is kEpsRay for all.
+    // [0] any-hit: origin + result index, direction + job (int bits); the value an unoccluded
+    //     ray adds is already in its result slot
+    // [1] closest-hit: origin + stop distance (a nearer hit ends the ray, emitter_span),
+    //     direction + tmax, value, meta = {result index, type | light << 2, pixel, job}
     float4* so[2];
     float4* sd[2];
-    float4* sv[2];
-    int4*   sm[2];
+    float4* sv;
+    int4*   sm;
     int64_t shadow_cap;
     // per-path radiance of path g at g % ring_size until its pixel resolves; per pixel
     // (at its first path's ring index) the count of its finished paths
@@ -132,7 +134,7 @@ constexpr int kAdjLog = 16;
 
 struct LaunchShape
 {
-    int grid_trace, grid_any, grid_connect, grid_shade, grid_regen, grid_small, block;  // grid_any: any-hit k_connect
+    int grid_trace, grid_any, grid_connect, grid_shade, grid_regen, grid_small, block;  // grid_any: k_shadow
     bool fast_only = false;  // every job traverses in FAST mode: kernels built without the REF traversal
     int  lights = 3;         // light kinds of the jobs (1 environment, 2 area, 3 both): the k_shade build
 };
