@@ -42,35 +42,81 @@ namespace mcrt {
 // ---------------------------------------------------------------------------
 // batch trace
 // ---------------------------------------------------------------------------
-// Each warp takes the next 32 consecutive rays from a counter until the batch is done (the
-// wavefront traversal kernels' warp batch fetch); STACK / MINB as the wavefront's builds:
-// 32-entry stacks when the tree is shallow enough, registers capped for MINB blocks per SM
-// in FAST mode (MODE 0, a build without the reference traversal), the general build in REF
-// mode (MODE 1).
+// FAST mode (MODE 0): trace_stream; STACK / MINB as the wavefront's builds, 32-entry stacks
+// when the tree is shallow enough, registers capped for MINB blocks per SM.  REF mode (MODE 1):
+// each warp takes the next 32 consecutive rays from a counter until the batch is done.
+struct BatchRays
+{
+    const SceneView&    s;
+    const float4*       rays;
+    float4*             hits;
+    int*                occ;
+    unsigned long long* counter;
+    bool                any;
+    __device__ __forceinline__ int take() const
+    {
+        return (threadIdx.x & 31) == 0 ? static_cast<int>(atomicAdd(counter, 32ull)) : 0;
+    }
+    __device__ __forceinline__ int share(int b) const { return __shfl_sync(0xffffffffu, b, 0); }
+    __device__ __forceinline__ const float4* src(int i, int k) const { return rays + 2 * static_cast<int64_t>(i) + k; }
+    __device__ __forceinline__ int begin(int i, float4 o4, float4 d4, float& tmin, float& tmax, float&,
+                                         const FastNode*& nodes, const float4*& tris) const
+    {
+        tmin = o4.w;
+        tmax = d4.w;
+        nodes = s.fast_nodes;
+        tris = s.fast_tris;
+        return i;
+    }
+    __device__ __forceinline__ void finish(int i, const FastTrav& r, const float4* tris, float dx, float dy,
+                                           float dz) const
+    {
+        if (any)
+            occ[i] = r.hit.prim >= 0 ? 1 : 0;
+        else if (r.hit.prim >= 0)
+        {
+            const Hit h = final_hit(r, tris, mk(dx, dy, dz));
+            hits[i] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+        }
+        else
+            hits[i] = make_float4(__int_as_float(0x7f800000), 0.f, 0.f, __int_as_float(-1));
+    }
+};
+
 template <bool ANY, int MODE, int STACK, int MINB>
 __global__ void __launch_bounds__(kTraceBlock, MINB)
-    k_trace(SceneView s, const float4* __restrict__ rays, int64_t n, float4* __restrict__ hits, int* __restrict__ occ,
+    k_trace(SceneView s, const float4* __restrict__ rays, int n, float4* __restrict__ hits, int* __restrict__ occ,
             int* err, unsigned long long* fetch)
 {
-    __shared__ int stack[STACK * kTraceBlock];
-    int*           st = stack + threadIdx.x;
-    const int      lane = threadIdx.x & 31;
-    while (true)
+    if constexpr (MODE == 0 && kStreamTraversal)
     {
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(fetch, 32ull);
-        b = __shfl_sync(0xffffffffu, b, 0);
-        if (b >= static_cast<unsigned long long>(n)) break;
-        const int64_t i = static_cast<int64_t>(b) + lane;
-        if (i >= n) continue;
-        float4 a = rays[2 * i], d = rays[2 * i + 1];
-        Hit    h;
-        bool any = trace_ray<ANY, STACK, false, MODE == 1>(s, MODE, xyz(a), xyz(d), a.w, d.w, st, kTraceBlock, h, err);
-        if (ANY)
-            occ[i] = any ? 1 : 0;
-        else
-            hits[i] = any ? make_float4(h.t, h.u, h.v, __int_as_float(h.prim))
-                          : make_float4(__int_as_float(0x7f800000), 0.f, 0.f, __int_as_float(-1));
+        __shared__ StreamSmem<STACK, kTraceBlock> sm;
+        BatchRays q{s, rays, hits, occ, fetch, ANY};
+        trace_stream<ANY, STACK, kTraceBlock, false, false>(q, n, sm, err, nullptr);
+    }
+    else
+    {
+        __shared__ int stack[STACK * kTraceBlock];
+        int*           st = stack + threadIdx.x;
+        const int      lane = threadIdx.x & 31;
+        while (true)
+        {
+            unsigned long long b = 0;
+            if (lane == 0) b = atomicAdd(fetch, 32ull);
+            b = __shfl_sync(0xffffffffu, b, 0);
+            if (b >= static_cast<unsigned long long>(n)) break;
+            const int64_t i = static_cast<int64_t>(b) + lane;
+            if (i >= n) continue;
+            float4 a = rays[2 * i], d = rays[2 * i + 1];
+            Hit    h;
+            bool   any =
+                trace_ray<ANY, STACK, false, MODE == 1>(s, MODE, xyz(a), xyz(d), a.w, d.w, st, kTraceBlock, h, err);
+            if (ANY)
+                occ[i] = any ? 1 : 0;
+            else
+                hits[i] = any ? make_float4(h.t, h.u, h.v, __int_as_float(h.prim))
+                              : make_float4(__int_as_float(0x7f800000), 0.f, 0.f, __int_as_float(-1));
+        }
     }
 }
 
@@ -499,25 +545,83 @@ __device__ __forceinline__ float4 hit_record(bool hit, const Hit& h)
     return hit ? make_float4(h.t, h.u, h.v, __int_as_float(h.prim)) : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
 }
 
+// trace_stream's batches of a wavefront queue: from a counter, or by the grid's stride
+struct QueueFetch
+{
+    int* counter;
+    int  base;  // first entry of this warp's next batch (grid stride)
+    bool batch;
+    __device__ __forceinline__ QueueFetch(int* c, bool batch_)
+        : counter(c), base(static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) & ~31u)), batch(batch_)
+    {
+    }
+    __device__ __forceinline__ int take()
+    {
+        if (batch) return (threadIdx.x & 31) == 0 ? atomicAdd(counter, 32) : 0;
+        const int b = base;
+        base += gridDim.x * blockDim.x;
+        return b;
+    }
+    __device__ __forceinline__ int share(int b) const { return __shfl_sync(0xffffffffu, b, 0); }
+};
+
+struct ExtendRays : QueueFetch
+{
+    const WaveArgs& a;
+    int             p;
+    __device__ __forceinline__ ExtendRays(const WaveArgs& a_, int p_)
+        : QueueFetch(&a_.ctrl->fetch[0], a_.batch_fetch != 0), a(a_), p(p_)
+    {
+    }
+    __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.qo[p][i] : &a.qd[p][i]; }
+    __device__ __forceinline__ int begin(int i, float4 o4, float4, float& tmin, float& tmax, float&,
+                                         const FastNode*& nodes, const float4*& tris) const
+    {
+        const SceneView& S = a.jobs[__float_as_int(o4.w)].scene;
+        tmin = kEpsRay;
+        tmax = __int_as_float(0x7f800000);
+        nodes = S.fast_nodes;
+        tris = S.fast_tris;
+        return i;
+    }
+    __device__ __forceinline__ void finish(int i, const FastTrav& r, const float4* tris, float dx, float dy,
+                                           float dz) const
+    {
+        const bool hit = r.hit.prim >= 0;
+        Hit        h;
+        if (hit) h = final_hit(r, tris, mk(dx, dy, dz));
+        __stcs(&a.hits[i], hit_record(hit, h));
+    }
+};
+
 template <int STACK, bool COUNT, int MINB, bool REFM = true>
 __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
 {
-    __shared__ int stack[STACK * kTraceBlock];
-    int*           st = stack + threadIdx.x;
-    const int      n = min(a.ctrl->qcount[p], static_cast<int>(a.capacity));
-    const float    inf = __int_as_float(0x7f800000);
-    TraceCount     cnt = {0u, 0u};
+    const int  n = min(a.ctrl->qcount[p], static_cast<int>(a.capacity));
+    TraceCount cnt = {0u, 0u};
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats[0], static_cast<unsigned long long>(n));
-    for (QueueWalk w(&a.ctrl->fetch[0], n, a.batch_fetch != 0); w.valid(); w.next())
+    if constexpr (!REFM && kStreamTraversal)
     {
-        const int i = w.i;
-        if (i >= n) continue;
-        float4        o = a.qo[p][i], d = a.qd[p][i];
-        const JobGPU& J = a.jobs[__float_as_int(o.w)];
-        Hit           h;
-        bool hit = trace_ray<false, STACK, COUNT, REFM>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay, inf, st,
-                                                        kTraceBlock, h, a.err, &cnt);
-        a.hits[i] = hit_record(hit, h);
+        __shared__ StreamSmem<STACK, kTraceBlock> sm;
+        ExtendRays                                q(a, p);
+        trace_stream<false, STACK, kTraceBlock, COUNT, false>(q, n, sm, a.err, &cnt);
+    }
+    else
+    {
+        __shared__ int stack[STACK * kTraceBlock];
+        int*           st = stack + threadIdx.x;
+        const float    inf = __int_as_float(0x7f800000);
+        for (QueueWalk w(&a.ctrl->fetch[0], n, a.batch_fetch != 0); w.valid(); w.next())
+        {
+            const int i = w.i;
+            if (i >= n) continue;
+            float4        o = a.qo[p][i], d = a.qd[p][i];
+            const JobGPU& J = a.jobs[__float_as_int(o.w)];
+            Hit           h;
+            bool hit = trace_ray<false, STACK, COUNT, REFM>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay, inf, st,
+                                                            kTraceBlock, h, a.err, &cnt);
+            a.hits[i] = hit_record(hit, h);
+        }
     }
     if (COUNT) flush_count(a.stats, 2, cnt);
 }
@@ -719,11 +823,13 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                 int k = base + __popc(live & lanemask_lt());
                 if (k < a.capacity)
                 {
-                    a.qo[pn][k] = make_float4(phit.x, phit.y, phit.z, __int_as_float(job));
-                    a.qd[pn][k] = make_float4(cdir.x, cdir.y, cdir.z, __int_as_float(pixel));
-                    a.qthr[pn][k] = make_float4(T2.x, T2.y, T2.z, __int_as_float(flags2 | (pend << 16)));
-                    a.qrad[pn][k] = rnew;
-                    a.qrng[pn][k] = rstate;
+                    // the queues are written and read once per iteration: streaming stores
+                    // leave the L2 to the tree (outdoor frame 84.6 -> 83.2 ms)
+                    __stcs(&a.qo[pn][k], make_float4(phit.x, phit.y, phit.z, __int_as_float(job)));
+                    __stcs(&a.qd[pn][k], make_float4(cdir.x, cdir.y, cdir.z, __int_as_float(pixel)));
+                    __stcs(&a.qthr[pn][k], make_float4(T2.x, T2.y, T2.z, __int_as_float(flags2 | (pend << 16))));
+                    __stcs(&a.qrad[pn][k], rnew);
+                    __stcs(reinterpret_cast<unsigned long long*>(&a.qrng[pn][k]), static_cast<unsigned long long>(rstate));
                     if (ADJ && nlog > 0)
                     {
                         a.qlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
@@ -784,15 +890,15 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                 }
                 if (qsel == 0)
                 {
-                    a.so[0][idx] = make_float4(phit.x, phit.y, phit.z, __int_as_float(dest + r));
-                    a.sd[0][idx] = make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, __int_as_float(job));
-                    a.nev[pn][dest + r] = nee[r].val;
+                    __stcs(&a.so[0][idx], make_float4(phit.x, phit.y, phit.z, __int_as_float(dest + r)));
+                    __stcs(&a.sd[0][idx], make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, __int_as_float(job)));
+                    __stcs(&a.nev[pn][dest + r], nee[r].val);
                 }
                 else
                 {
                     // .w: where a closest-hit ray stops at a nearer hit (tmin is kEpsRay for all)
-                    a.so[1][idx] = make_float4(phit.x, phit.y, phit.z, nee[r].tterm);
-                    a.sd[1][idx] = make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, nee[r].tmax);
+                    __stcs(&a.so[1][idx], make_float4(phit.x, phit.y, phit.z, nee[r].tterm));
+                    __stcs(&a.sd[1][idx], make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, nee[r].tmax));
                     a.sv[idx] = nee[r].val;
                     a.sm[idx] = make_int4(dest + r, nee[r].type | (nee[r].light << 2), pixel, job);
                 }
@@ -829,51 +935,127 @@ __device__ __forceinline__ void connect_result(const WaveArgs& a, const Grads& G
 // unoccluded ray adds to the slot its path will read; an occluded ray clears the slot.  So a
 // queue entry is a ray with its slot and job, 32 B instead of 64, and a ray that gets through
 // writes nothing; with the value and the kinds of result out of the kernel it holds fewer
-// registers beside the traversal's (no spills at 48; 12 blocks per SM as before).  Adjoint
+// registers beside the traversal's.  Adjoint
 // and forward run the same kernel: an environment ray has no emission derivative.
+struct ShadowRays : QueueFetch
+{
+    const WaveArgs& a;
+    int             p;
+    __device__ __forceinline__ ShadowRays(const WaveArgs& a_, int p_)
+        : QueueFetch(&a_.ctrl->fetch[1], a_.batch_fetch != 0), a(a_), p(p_)
+    {
+    }
+    __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.so[0][i] : &a.sd[0][i]; }
+    __device__ __forceinline__ int begin(int, float4 o4, float4 d4, float& tmin, float& tmax, float&,
+                                         const FastNode*& nodes, const float4*& tris) const
+    {
+        const SceneView& S = a.jobs[__float_as_int(d4.w)].scene;
+        tmin = kEpsRay;
+        tmax = __int_as_float(0x7f800000);
+        nodes = S.fast_nodes;
+        tris = S.fast_tris;
+        return __float_as_int(o4.w);
+    }
+    __device__ __forceinline__ void finish(int dest, const FastTrav& r, const float4*, float, float, float) const
+    {
+        if (r.hit.prim >= 0) a.nev[p ^ 1][dest] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+};
+
 template <int STACK, bool COUNT, int MINB, bool REFM = true>
 __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kAnyHitMinBlocks : MINB) k_shadow(WaveArgs a, int p)
 {
-    __shared__ int stack[STACK * kTraceBlock];
-    int*           st = stack + threadIdx.x;
-    TraceCount     cnt = {0u, 0u};
-    const int      n = min(a.ctrl->scount[0], static_cast<int>(a.shadow_cap));
+    TraceCount cnt = {0u, 0u};
+    const int  n = min(a.ctrl->scount[0], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
-    for (QueueWalk w(&a.ctrl->fetch[1], n, a.batch_fetch != 0); w.valid(); w.next())
+    if constexpr (!REFM && kStreamTraversal)
     {
-        const int k = w.i;
-        if (k >= n) continue;
-        const float4  o = a.so[0][k], d = a.sd[0][k];
-        const JobGPU& J = a.jobs[__float_as_int(d.w)];
-        Hit           h;
-        if (trace_ray<true, STACK, COUNT, REFM>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay,
-                                                __int_as_float(0x7f800000), st, kTraceBlock, h, a.err, &cnt))
-            a.nev[p ^ 1][__float_as_int(o.w)] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __shared__ StreamSmem<STACK, kTraceBlock> sm;
+        ShadowRays                                q(a, p);
+        trace_stream<true, STACK, kTraceBlock, COUNT, false>(q, n, sm, a.err, &cnt);
+    }
+    else
+    {
+        __shared__ int stack[STACK * kTraceBlock];
+        int*           st = stack + threadIdx.x;
+        for (QueueWalk w(&a.ctrl->fetch[1], n, a.batch_fetch != 0); w.valid(); w.next())
+        {
+            const int k = w.i;
+            if (k >= n) continue;
+            const float4  o = a.so[0][k], d = a.sd[0][k];
+            const JobGPU& J = a.jobs[__float_as_int(d.w)];
+            Hit           h;
+            if (trace_ray<true, STACK, COUNT, REFM>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay,
+                                                    __int_as_float(0x7f800000), st, kTraceBlock, h, a.err, &cnt))
+                a.nev[p ^ 1][__float_as_int(o.w)] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     if (COUNT) flush_count(a.stats, 4, cnt);
 }
 
 // the bounded closest-hit queue (next-event rays to area lights)
+template <bool ADJ>
+struct ConnectRays : QueueFetch
+{
+    const WaveArgs& a;
+    const Grads&    G;
+    int             p;
+    __device__ __forceinline__ ConnectRays(const WaveArgs& a_, const Grads& G_, int p_)
+        : QueueFetch(&a_.ctrl->fetch[2], a_.batch_fetch != 0), a(a_), G(G_), p(p_)
+    {
+    }
+    __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.so[1][i] : &a.sd[1][i]; }
+    __device__ __forceinline__ int begin(int k, float4 o4, float4 d4, float& tmin, float& tmax, float& tterm,
+                                         const FastNode*& nodes, const float4*& tris) const
+    {
+        const SceneView& S = a.jobs[a.sm[k].w].scene;
+        tmin = kEpsRay;
+        tmax = d4.w;
+        tterm = o4.w;
+        nodes = S.fast_nodes;
+        tris = S.fast_tris;
+        return k;
+    }
+    __device__ __forceinline__ void finish(int k, const FastTrav& r, const float4* tris, float dx, float dy,
+                                           float dz) const
+    {
+        const float3 d = mk(dx, dy, dz);
+        const bool   hit = r.hit.prim >= 0 && !(r.best < r.tterm);
+        Hit          h;
+        if (hit) h = final_hit(r, tris, d);
+        connect_result<ADJ>(a, G, p, k, d, hit, h);
+    }
+};
+
 template <int STACK, bool COUNT, int MINB, bool ADJ, bool REFM = true>
-__global__ void __launch_bounds__(kTraceBlock, MINB) k_connect(WaveArgs a, int p)
+__global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kConnectMinBlocks : MINB) k_connect(WaveArgs a, int p)
 {
     extern __shared__ float sgrad[];
-    __shared__ int stack[STACK * kTraceBlock];
-    const Grads    G = grads_begin<ADJ, GRAD_EMISSION>(a, sgrad);
-    int*           st = stack + threadIdx.x;
-    TraceCount     cnt = {0u, 0u};
-    const int      n = min(a.ctrl->scount[1], static_cast<int>(a.shadow_cap));
+    const Grads             G = grads_begin<ADJ, GRAD_EMISSION>(a, sgrad);
+    TraceCount              cnt = {0u, 0u};
+    const int               n = min(a.ctrl->scount[1], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
-    for (QueueWalk w(&a.ctrl->fetch[2], n, a.batch_fetch != 0); w.valid(); w.next())
+    if constexpr (!REFM && kStreamTraversal)
     {
-        const int k = w.i;
-        if (k >= n) continue;
-        const float4  o = a.so[1][k], d = a.sd[1][k];
-        const JobGPU& J = a.jobs[a.sm[k].w];
-        Hit           h;
-        bool hit = trace_ray<false, STACK, COUNT, REFM, true>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay, d.w, st,
-                                                              kTraceBlock, h, a.err, &cnt, o.w);
-        connect_result<ADJ>(a, G, p, k, xyz(d), hit, h);
+        __shared__ StreamSmem<STACK, kTraceBlock> sm;
+        ConnectRays<ADJ>                          q(a, G, p);
+        trace_stream<false, STACK, kTraceBlock, COUNT, true>(q, n, sm, a.err, &cnt);
+    }
+    else
+    {
+        __shared__ int stack[STACK * kTraceBlock];
+        int*           st = stack + threadIdx.x;
+        for (QueueWalk w(&a.ctrl->fetch[2], n, a.batch_fetch != 0); w.valid(); w.next())
+        {
+            const int k = w.i;
+            if (k >= n) continue;
+            const float4  o = a.so[1][k], d = a.sd[1][k];
+            const JobGPU& J = a.jobs[a.sm[k].w];
+            Hit           h;
+            const bool hit = trace_ray<false, STACK, COUNT, REFM, true>(J.scene, J.traverse, xyz(o), xyz(d), kEpsRay,
+                                                                        d.w, st, kTraceBlock, h, a.err, &cnt, o.w);
+            connect_result<ADJ>(a, G, p, k, xyz(d), hit, h);
+        }
     }
     if (COUNT) flush_count(a.stats, 4, cnt);
     grads_end<ADJ, GRAD_EMISSION>(a, sgrad);
@@ -2188,41 +2370,35 @@ void enqueue_render_begin(const WaveArgs& a, bool waves, int64_t limit, cudaStre
 
 LaunchShape launch_shape() { return launch_shape_variant(false, false); }
 
+namespace {
+template <int STACK, int MINB, bool REFM>
+void traversal_occupancy(int& extend, int& shadow, int& connect)
+{
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&extend, k_extend<STACK, false, MINB, REFM>, kTraceBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadow, k_shadow<STACK, false, MINB, REFM>, kTraceBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&connect, k_connect<STACK, false, MINB, false, REFM>, kTraceBlock, 0);
+}
+}  // namespace
+
 LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only)
 {
-    LaunchShape ls;
-    int         sms = num_sms();
-    int         occ_t = 0, occ_s = 0, occ_a = 0;
+    LaunchShape   ls;
+    const int     sms = num_sms();
+    int           occ_t = 0, occ_a = 0, occ_c = 0, occ_s = 0;
     constexpr int B = kTraceMinBlocks;
     if (!fast_only)  // the general build (see with_variant)
-    {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_extend<kStack, false, 1, true>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_shadow<kStack, false, 1, true>, kTraceBlock, 0);
-    }
+        traversal_occupancy<kStack, 1, true>(occ_t, occ_a, occ_c);
     else if (stack32)
-    {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &occ_t, regcap ? k_extend<kSmallStack, false, B, false> : k_extend<kSmallStack, false, 1, false>,
-            kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &occ_a,
-            regcap ? k_shadow<kSmallStack, false, B, false> : k_shadow<kSmallStack, false, 1, false>,
-            kTraceBlock, 0);
-    }
+        regcap ? traversal_occupancy<kSmallStack, B, false>(occ_t, occ_a, occ_c)
+               : traversal_occupancy<kSmallStack, 1, false>(occ_t, occ_a, occ_c);
     else
-    {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &occ_t, regcap ? k_extend<kStack, false, B, false> : k_extend<kStack, false, 1, false>, kTraceBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &occ_a,
-            regcap ? k_shadow<kStack, false, B, false> : k_shadow<kStack, false, 1, false>,
-            kTraceBlock, 0);
-    }
+        regcap ? traversal_occupancy<kStack, B, false>(occ_t, occ_a, occ_c)
+               : traversal_occupancy<kStack, 1, false>(occ_t, occ_a, occ_c);
     ls.fast_only = fast_only;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_shade<false>, 128, 0);
     ls.grid_trace = sms * std::max(occ_t, 1);
     ls.grid_any = sms * std::max(occ_a, 1);
-    ls.grid_connect = ls.grid_trace;
+    ls.grid_connect = sms * std::max(occ_c, 1);
     ls.grid_shade = sms * std::max(occ_s, 1);
     ls.grid_regen = ls.grid_shade;
     ls.grid_small = sms * 8;
@@ -2600,12 +2776,21 @@ static int trace_impl(mcrt_scene* s, const mcrt_ray* rays, int64_t n, void* out,
     float4*             hits = static_cast<float4*>(d_out);
     int*                o = static_cast<int*>(d_out);
     const bool          small = stack_depth(s, traverse) + 2 < kSmallStack;
+    // 2^30 rays per launch: the kernels count rays in 32 bits
+    constexpr int64_t kSlice = int64_t(1) << 30;
     auto launch = [&](auto kernel) {
         int occ = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kTraceBlock, 0);
-        const int64_t want = (n + kTraceBlock - 1) / kTraceBlock;
-        const int grid = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(num_sms()) * std::max(occ, 1)));
-        kernel<<<grid, kTraceBlock, 0, st>>>(s->view, d_rays, n, hits, o, d_err, d_fetch);
+        for (int64_t off = 0; off < n; off += kSlice)
+        {
+            const int64_t m = std::min(n - off, kSlice);
+            if (off > 0) cudaMemsetAsync(d_fetch, 0, sizeof(*d_fetch), st);
+            const int64_t want = (m + kTraceBlock - 1) / kTraceBlock;
+            const int     grid =
+                static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(num_sms()) * std::max(occ, 1)));
+            kernel<<<grid, kTraceBlock, 0, st>>>(s->view, d_rays + 2 * off, static_cast<int>(m), any ? nullptr : hits + off,
+                                                 any ? o + off : nullptr, d_err, d_fetch);
+        }
     };
     if (traverse == MCRT_TRAVERSE_REF)
         any ? launch(k_trace<true, 1, kStack, 1>) : launch(k_trace<false, 1, kStack, 1>);

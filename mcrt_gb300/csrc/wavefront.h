@@ -33,22 +33,15 @@ constexpr int kTraceBlock = 128;
 constexpr int kStack = 64;
 // the smaller traversal stack, used when the tree is shallow enough (MCRT_VARIANT_STACK32)
 constexpr int kSmallStack = 32;
-// Traversal kernels under MCRT_VARIANT_REGCAP: __launch_bounds__(kTraceBlock, kTraceMinBlocks)
-// caps them at 56 registers, so 9 blocks (36 warps) fit an SM.  Measured on the cfg1 frame:
-// 8 blocks (64 registers) 52.6 / 59.9 ms extend / connect, 9 blocks 52.2 / 56.7, 10 blocks
-// (48 registers, spills) 54.4 / 57.0.
-#ifndef MCRT_TRACE_MIN_BLOCKS
-#define MCRT_TRACE_MIN_BLOCKS 9
-#endif
-constexpr int kTraceMinBlocks = MCRT_TRACE_MIN_BLOCKS;
-// The any-hit next-event kernel under MCRT_VARIANT_REGCAP: 40 registers, 12 blocks per SM
-// (40 B of spills).  Next-event stage per cfg1 frame: 10 blocks (48 registers, no spills)
-// 33.96 ms, 12 blocks 32.53 (an earlier build, with tmin read from the queue and more
-// spills: 9 blocks 37.5, 10 blocks 36.5, 12 blocks 38.8).
-#ifndef MCRT_ANYHIT_MIN_BLOCKS
-#define MCRT_ANYHIT_MIN_BLOCKS 12
-#endif
-constexpr int kAnyHitMinBlocks = MCRT_ANYHIT_MIN_BLOCKS;
+// Blocks of kTraceBlock threads per SM that the traversal kernels' registers are capped for
+// under MCRT_VARIANT_REGCAP.  Outdoor frame (1.3 M triangles, 67 M paths), extension /
+// next-event ms: extension rays at 9 blocks (56 registers) 38.9, at 8 (64, no spills) 37.7,
+// at 7 39.9; next-event rays to the environment at 12 (40 registers, spills) 27.6, at 10 (48)
+// 23.3, at 9 23.5.  With the lanes refilled (trace_stream) more warps than this no longer help.
+// Next-event rays to area lights: 7 blocks (72 registers) 0.68 ms per Cornell frame, 8 0.72.
+constexpr int kTraceMinBlocks = 8;
+constexpr int kConnectMinBlocks = 7;
+constexpr int kAnyHitMinBlocks = 10;
 constexpr int kMaxDepth = 62;
 constexpr int64_t kMaxQueue = int64_t(1) << 27;     // rays per queue (result indices stay in int)
 // Streaming schedule default: 64 M rays (49 GB of queues).  Per cfg1 frame (67 M paths):

@@ -1,0 +1,58 @@
+"""The streamed traversal: a ray's answer does not depend on the batch it is traced in, on its
+place in the batch or on which lane took it, so every batch size must give, ray by ray, the
+bits of any other; closest-hit and any-hit queries of one ray agree on whether it hits."""
+import numpy as np
+import pytest
+
+from conftest import golden
+from parity import classify
+
+pytestmark = pytest.mark.gpu
+
+# one ray, a warp's batch and its edges, a block, more batches than a block has warps, ragged
+SIZES = [1, 2, 31, 32, 33, 127, 128, 129, 1023, 20011]
+
+
+def _rays(n):
+    """Rays of very different lengths side by side: incoherent, short segments, misses, an
+    axis-parallel direction, a direction that is not normalised."""
+    rng = np.random.default_rng(11)
+    r = np.zeros((n, 8), np.float32)
+    r[:, 0:3] = rng.uniform(-1.5, 1.5, (n, 3))
+    d = rng.normal(size=(n, 3))
+    r[:, 4:7] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    r[:, 3], r[:, 7] = 1e-4, 1e30
+    r[1::7, 7] = 0.05
+    r[2::7, 0:3] += 50.0
+    r[3::7, 4:7] = (0.0, -1.0, 0.0)
+    r[4::7, 4:7] *= 3.0
+    return r
+
+
+@pytest.fixture(scope="module")
+def scene(cuda_device):
+    from mcrt_gb300 import GpuScene, scenes
+    return GpuScene(scenes.cfg1_scene(level=5))
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_batch_size_and_order_change_no_ray(n, scene):
+    rays = _rays(SIZES[-1])
+    whole = scene.trace_closest(rays)
+    occ = scene.trace_any(rays)
+    assert np.array_equal(occ != 0, whole[:, 3].view(np.int32) >= 0)
+    order = np.random.default_rng(n).permutation(rays.shape[0])[:n]
+    part = scene.trace_closest(rays[order])
+    assert np.array_equal(part.view(np.int32), whole[order].view(np.int32))
+    assert np.array_equal(scene.trace_any(rays[order]), occ[order])
+
+
+def test_streamed_hits_match_the_reference_tree(cuda_device):
+    """Against SplitBVH's own hits, by the parity rule of the other traversal tests."""
+    from parity import fixture_scene
+    from mcrt_gb300 import GpuScene
+    fx = golden("ref_traverse_sphere5.npz")
+    out = GpuScene(fixture_scene(fx)).trace_closest(fx["rays_bounce"])
+    bad, _ = classify(fx["verts"], fx["rays_bounce"], fx["t_bounce"], fx["prim_bounce"], out[:, 0],
+                      out[:, 3].view(np.int32))
+    assert not bad.any()
