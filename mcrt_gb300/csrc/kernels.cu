@@ -2576,6 +2576,33 @@ int validate_job(const mcrt_scene* s, const mcrt_camera* c, const mcrt_render_pa
 
 int set_error(int code, const std::string& msg) { return fail(code, msg); }
 
+namespace {
+struct ThreadScratch
+{
+    void*  ptr = nullptr;
+    size_t bytes = 0;
+    ~ThreadScratch()
+    {
+        if (ptr) cudaFree(ptr);  // at thread exit (an error after the runtime is gone is ignored)
+    }
+};
+}  // namespace
+
+void* thread_scratch(int device, size_t bytes, bool& failed)
+{
+    constexpr int              kDevices = 64;
+    thread_local ThreadScratch buffers[kDevices];
+    failed = false;
+    if (device < 0 || device >= kDevices || bytes > kThreadScratchMax) return nullptr;
+    ThreadScratch& b = buffers[device];
+    if (!b.ptr && cudaMalloc(&b.ptr, kThreadScratchMax) != cudaSuccess)
+    {
+        b.ptr = nullptr;
+        failed = true;
+    }
+    return b.ptr;
+}
+
 bool fast_layout_wide() { return MCRT_FAST_WIDE != 0; }
 
 const SceneView& scene_view(const mcrt_scene* s) { return s->view; }
@@ -2671,27 +2698,6 @@ int mcrt_scene_set_materials(mcrt_scene* s, int32_t n, const mcrt_material* m, v
     return MCRT_OK;
 }
 
-// Device buffer of the host-buffer trace calls of one host thread on one device, kept for
-// the thread's life (1 MB: up to about 20,000 rays per call).
-constexpr size_t kThreadTraceBufferMax = size_t(1) << 20;
-struct ThreadTraceBuffer
-{
-    void*  ptr = nullptr;
-    size_t bytes = 0;
-    ~ThreadTraceBuffer()
-    {
-        if (ptr) cudaFree(ptr);  // at thread exit (an error after the runtime is gone is ignored)
-    }
-};
-
-// this thread's buffer for `device`, or null (device index past the table: no reuse)
-ThreadTraceBuffer* thread_trace_buffer(int device)
-{
-    constexpr int                  kDevices = 64;
-    thread_local ThreadTraceBuffer buffers[kDevices];
-    return device >= 0 && device < kDevices ? &buffers[device] : nullptr;
-}
-
 static int trace_impl(mcrt_scene* s, const mcrt_ray* rays, int64_t n, void* out, bool any, int32_t traverse,
                       int32_t ptr_mode, void* stream)
 {
@@ -2723,20 +2729,15 @@ static int trace_impl(mcrt_scene* s, const mcrt_ray* rays, int64_t n, void* out,
         // per call
         const size_t rays_bytes = (sizeof(mcrt_ray) * n + 15) & ~static_cast<size_t>(15);
         const size_t need = rays_bytes + status_off + sizeof(TraceStatus);
-        ThreadTraceBuffer* tb = thread_trace_buffer(s->device);
-        if (tb && need <= kThreadTraceBufferMax)
+        bool         failed = false;
+        if (void* kept = thread_scratch(s->device, need, failed))
         {
-            if (tb->bytes < need)
-            {
-                if (cudaMalloc(&tb->ptr, kThreadTraceBufferMax) != cudaSuccess)
-                {
-                    tb->ptr = nullptr;
-                    return fail(MCRT_ERR_OUT_OF_MEMORY, "trace buffer allocation failed");
-                }
-                tb->bytes = kThreadTraceBufferMax;
-            }
-            tmp_rays = tb->ptr;
-            tmp_out = static_cast<char*>(tb->ptr) + rays_bytes;
+            tmp_rays = kept;
+            tmp_out = static_cast<char*>(kept) + rays_bytes;
+        }
+        else if (failed)
+        {
+            return fail(MCRT_ERR_OUT_OF_MEMORY, "trace buffer allocation failed");
         }
         else
         {

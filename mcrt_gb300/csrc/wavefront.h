@@ -171,6 +171,12 @@ void enqueue_wave_plain(const WaveArgs& a, int max_depth, const LaunchShape& ls,
 CameraGPU make_camera(const mcrt_camera& c);
 // argument checks shared by the render entry points; sets the last error
 int validate_job(const mcrt_scene* s, const mcrt_camera* c, const mcrt_render_params* p);
+// Device memory of one host thread on one device, kept for the thread's life: small requests of
+// calls that return only when their work is done (host-buffer traces, film sums) pay no
+// cudaMalloc / cudaFree (which synchronises the device).  Null when `bytes` is over the limit
+// or the device index past the table (allocate instead), or when its allocation failed.
+constexpr size_t kThreadScratchMax = size_t(1) << 20;
+void* thread_scratch(int device, size_t bytes, bool& failed);
 // records the calling thread's last error message and returns `code`
 int set_error(int code, const std::string& msg);
 // read-only facts about a scene handle
