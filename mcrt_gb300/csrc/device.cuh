@@ -160,7 +160,11 @@ MCRT_HDI float3 operator-(float3 a, float3 b) { return mk(a.x - b.x, a.y - b.y, 
 MCRT_HDI float3 operator*(float3 a, float3 b) { return mk(a.x * b.x, a.y * b.y, a.z * b.z); }
 MCRT_HDI float3 operator*(float3 a, float s) { return mk(a.x * s, a.y * s, a.z * s); }
 MCRT_HDI float3 operator-(float3 a) { return mk(-a.x, -a.y, -a.z); }
-__device__ __forceinline__ float  dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// The multiply-adds of sums of products are written out where the compiler could choose which
+// product it rounds first: it chose differently for two copies of one expression in different
+// surroundings, and an image must not change in its last bits because code around it does.
+__device__ __forceinline__ float dot3(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.x, b.x, a.y * b.y)); }
+__device__ __forceinline__ float dot_yx(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
 __device__ __forceinline__ float3 cross3(float3 a, float3 b)
 {
     return mk(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
@@ -187,16 +191,21 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x)
     return x ^ (x >> 31);
 }
 
+constexpr uint64_t kPcgMul = 6364136223846793005ull;
 struct Pcg
 {
     uint64_t state, inc;
     __device__ __forceinline__ uint32_t next()
     {
         uint64_t old = state;
-        state = old * 6364136223846793005ull + inc;
+        state = old * kPcgMul + inc;
+        return output(old);
+    }
+    static __device__ __forceinline__ uint32_t output(uint64_t old)
+    {
         uint32_t xs = static_cast<uint32_t>(((old >> 18u) ^ old) >> 27u);
         uint32_t rot = static_cast<uint32_t>(old >> 59u);
-        return (xs >> rot) | (xs << ((32u - rot) & 31u));
+        return __funnelshift_r(xs, xs, rot);
     }
     __device__ __forceinline__ float uniform() { return static_cast<float>(next() >> 8) * (1.0f / 16777216.0f); }
     __device__ __forceinline__ void seed(uint64_t seed, uint32_t pixel, uint32_t sample)
@@ -216,6 +225,60 @@ enum Dim
     D_ENV_LIGHT_0 = 0, D_ENV_LIGHT_1, D_ENV_JITTER_U, D_ENV_JITTER_V, D_ENV_BSDF_0, D_ENV_BSDF_1,
     D_AREA_BSDF_0, D_AREA_BSDF_1, D_LIGHT_PICK, D_LIGHT_U, D_LIGHT_V, D_CONT_0, D_CONT_1, D_RR,
     NUM_DIMS
+};
+
+// The generator's state k draws on is state * kPcgMul^k + inc * (1 + ... + kPcgMul^(k-1)).
+template <int K>
+struct PcgSkip
+{
+    static constexpr uint64_t mul = PcgSkip<K - 1>::mul * kPcgMul, add = PcgSkip<K - 1>::add * kPcgMul + 1ull;
+};
+template <>
+struct PcgSkip<0>
+{
+    static constexpr uint64_t mul = 1ull, add = 0ull;
+};
+
+// A vertex's NUM_DIMS numbers, as an array (ArrayDraws) or each made where it is used from the
+// generator's state at the vertex (VertexDraws): a mirror or dielectric vertex uses one or two of
+// the fourteen, a Lambert one under an environment nine, and no array lies in local memory.
+struct ArrayDraws
+{
+    const float* u;
+    template <int K>
+    __device__ __forceinline__ float at() const
+    {
+        return u[K];
+    }
+    template <int K>
+    __device__ __forceinline__ float2 pair() const
+    {
+        return make_float2(u[K], u[K + 1]);
+    }
+};
+struct VertexDraws
+{
+    uint64_t state, inc;
+    template <int K>
+    __device__ __forceinline__ float at() const
+    {
+        const uint64_t at = state * PcgSkip<K>::mul + inc * PcgSkip<K>::add;
+        return number(at);
+    }
+    template <int K>
+    __device__ __forceinline__ float2 pair() const  // numbers K and K + 1
+    {
+        const uint64_t at = state * PcgSkip<K>::mul + inc * PcgSkip<K>::add;
+        return make_float2(number(at), number(at * kPcgMul + inc));
+    }
+    static __device__ __forceinline__ float number(uint64_t at)
+    {
+        return static_cast<float>(Pcg::output(at) >> 8) * (1.0f / 16777216.0f);
+    }
+    __device__ __forceinline__ uint64_t after() const  // the generator's state after the vertex
+    {
+        return state * PcgSkip<NUM_DIMS>::mul + inc * PcgSkip<NUM_DIMS>::add;
+    }
 };
 
 // ---------------------------------------------------------------------------
@@ -1076,10 +1139,14 @@ struct Frame
         z = n;
     }
     __device__ __forceinline__ float3 to_world(float3 c) const { return x * c.x + y * c.y + z * c.z; }
+    // dot3 and dot_yx: the roundings of a sampled and of the incoming direction (see dot3)
     __device__ __forceinline__ float3 to_local(float3 v) const { return mk(dot3(v, x), dot3(v, y), dot3(v, z)); }
+    __device__ __forceinline__ float3 in_local(float3 v) const { return mk(dot_yx(v, x), dot_yx(v, y), dot_yx(v, z)); }
 };
 
-__device__ __forceinline__ float3 reflect_world(float3 wi, float3 n) { return n * (2.0f * dot3(n, wi)) - wi; }
+// the reflection of wi about n, given n . wi
+__device__ __forceinline__ float3 reflect_by(float3 wi, float3 n, float nw) { return n * (2.0f * nw) - wi; }
+__device__ __forceinline__ float3 reflect_world(float3 wi, float3 n) { return reflect_by(wi, n, dot3(n, wi)); }
 
 // fresnelReflectance (geometry.cpp:14-43)
 __device__ __forceinline__ float fresnel(float cos_i, float ior)
@@ -1176,7 +1243,7 @@ __device__ __forceinline__ BsdfSample bsdf_sample(const Mat& m, float3 wi, float
     s.pdf = 0.f;
     if (m.type == MAT_SPEC)
     {
-        s.wo = reflect_world(wi, nl);
+        s.wo = reflect_by(wi, nl, dot_yx(nl, wi));
         s.weight = m.color;
         s.pdf = 1.f;
     }
@@ -1184,7 +1251,9 @@ __device__ __forceinline__ BsdfSample bsdf_sample(const Mat& m, float3 wi, float
     {
         bool   outside = dot3(wi, nl) > 0.f;
         float3 n = outside ? nl : -nl;
-        float3 refl = normalize3(reflect_world(wi, n));
+        // (products and sums in the order and with the roundings of the parity images, see dot3)
+        const float cw = __fadd_rn(fmaf(n.y, wi.y, __fmul_rn(n.x, wi.x)), __fmul_rn(n.z, wi.z));
+        float3      refl = normalize3(reflect_by(wi, n, cw));
         float  nc = 1.f, nt = m.ior;
         float  nnt = outside ? nc / nt : nt / nc;
         float  ddn = dot3(-wi, n);
@@ -1197,7 +1266,9 @@ __device__ __forceinline__ BsdfSample bsdf_sample(const Mat& m, float3 wi, float
         }
         else
         {
-            float3 tdir = normalize3(-wi * nnt - n * (ddn * nnt + sqrtf(cos2t)));
+            const float k = fmaf(ddn, nnt, sqrtf(cos2t));
+            float3      tdir = normalize3(mk(fmaf(-n.x, k, -wi.x * nnt), fmaf(-n.y, k, -wi.y * nnt),
+                                        fmaf(-n.z, k, -wi.z * nnt)));
             float  Re = fresnel(dot3(wi, nl), nt / nc);
             float  Tr = 1.f - Re;
             float  P = Re;
@@ -1223,7 +1294,7 @@ __device__ __forceinline__ BsdfSample bsdf_sample(const Mat& m, float3 wi, float
     {
         float3 n = dot3(wi, nl) < 0.f ? -nl : nl;
         Frame  fr(n);
-        float3 wl = fr.to_local(wi);
+        float3 wl = fr.in_local(wi);
         float  a = m.roughness;
         s.wo = n;
         s.weight = mk(0.f, 0.f, 0.f);
@@ -1234,9 +1305,10 @@ __device__ __forceinline__ BsdfSample bsdf_sample(const Mat& m, float3 wi, float
             float3 t1 = lensq > 0.f ? mk(-vh.y, vh.x, 0.f) * rsqrtf(lensq) : mk(1.f, 0.f, 0.f);
             float3 t2 = cross3(vh, t1);
             float  r = sqrtf(r1);
-            float  phi = 2.f * kPi * r2;
-            float  p1 = r * cosf(phi);
-            float  p2 = r * sinf(phi);
+            float  phi = 2.f * kPi * r2, sphi, cphi;
+            sincosf(phi, &sphi, &cphi);
+            float p1 = r * cphi;
+            float p2 = r * sphi;
             float  sh = 0.5f * (1.f + vh.z);
             p2 = (1.f - sh) * sqrtf(fmaxf(0.f, 1.f - p1 * p1)) + sh * p2;
             float3 nh = t1 * p1 + t2 * p2 + vh * sqrtf(fmaxf(0.f, 1.f - p1 * p1 - p2 * p2));
@@ -1254,8 +1326,9 @@ __device__ __forceinline__ BsdfSample bsdf_sample(const Mat& m, float3 wi, float
     else  // DIFF (and any other type, as Material's default)
     {
         float  x = r1 * (2.f * kPi);
-        float  r2s = sqrtf(r2);
-        float3 c = mk(cosf(x) * r2s, sinf(x) * r2s, sqrtf(1.f - r2));
+        float  r2s = sqrtf(r2), sx, cx;
+        sincosf(x, &sx, &cx);  // the bits of sinf and cosf (every float in [0, 8) compared), one reduction
+        float3 c = mk(cx * r2s, sx * r2s, sqrtf(1.f - r2));
         Frame  onb(nl);
         float3 wo = onb.to_world(c);
         float  c_o = fmax_ref(dot3(wo, nl), kEpsCos);
@@ -1275,7 +1348,7 @@ __device__ __forceinline__ float bsdf_pdf(const Mat& m, float3 wi, float3 nl, fl
     {
         float3 n = dot3(wi, nl) < 0.f ? -nl : nl;
         Frame  fr(n);
-        float3 wl = fr.to_local(wi), ol = fr.to_local(wo);
+        float3 wl = fr.in_local(wi), ol = fr.to_local(wo);
         if (wl.z <= 0.f || ol.z <= 0.f) return 0.f;
         float3 h = normalize3(wl + ol);
         return ggx_G1(wl, m.roughness) * ggx_D(h, m.roughness) / (4.f * wl.z);
@@ -1292,7 +1365,7 @@ __device__ __forceinline__ float3 bsdf_eval(const Mat& m, float3 wi, float3 nl, 
     {
         float3 n = dot3(wi, nl) < 0.f ? -nl : nl;
         Frame  fr(n);
-        float3 wl = fr.to_local(wi), ol = fr.to_local(wo);
+        float3 wl = fr.in_local(wi), ol = fr.to_local(wo);
         if (wl.z <= 0.f || ol.z <= 0.f) return mk(0.f, 0.f, 0.f);
         float3 h = normalize3(wl + ol);
         float  a = m.roughness;
@@ -1380,8 +1453,10 @@ __device__ __forceinline__ void env_sample(const SceneView& s, float r1, float r
     int   vi = clampi(static_cast<int>(v * static_cast<float>(H)), 0, H - 1);
     float phi = v * kPi;
     float theta = u * 2.f * kPi;
-    float sp = sinf(phi);
-    dir = mk(sp * sinf(theta), cosf(phi), sp * -cosf(theta));
+    float sp, cp, st, ct;
+    sincosf(phi, &sp, &cp);
+    sincosf(theta, &st, &ct);
+    dir = mk(sp * st, cp, sp * -ct);
     pdf = env_pdf_at(s, ui, vi);
     rad = xyz(__ldg(&s.env_rgb[ui + vi * W]));
 }

@@ -629,12 +629,22 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
 // Adjoint (ADJ): emission derivatives at emitter hits (the coefficient of E), and at a
 // parameterised Lambert vertex k the - dL/dI * L_before(k) / albedo_k half of the albedo
 // derivative; the vertex's material id goes to the path's log for the other half.
-// Registers capped at 56 (9 blocks per SM).  Per cfg1 frame: uncapped (80 registers)
-// 32.4 ms, 8 blocks 26.5, 9 blocks 25.0, 10 blocks 26.3.  One build only: builds under
-// different register budgets contract multiply-adds differently, and every
-// configuration must render the same image.
+//
+// What bounds it: the latency of scattered reads (hit normals, materials, environment tables:
+// 9-12 of 19 stall cycles per issue, DRAM 26-34 % busy) and, with an environment, the
+// instruction cache.  The continuation is sampled first, so that the path's place in the next
+// queue, and with it the place of its next-event results, is known before the next-event rays
+// are made: each ray is written to its queue as it is made (an array of up to four lay in local
+// memory before, with the vertex's 14 random numbers), and a number is drawn where it is used
+// (VertexDraws).  Outdoor frame 18.7 -> 16.1 ms of shading (67 M paths; sincosf for the sine and
+// cosine of one angle is 0.7 of that), a 512x512 Cornell frame with 256 albedos forward and
+// adjoint 24.7 -> 23.5 ms.
+// Registers: environment-only build at 7 / 8 / 9 / 10 blocks per SM 17.6 / 16.8 / 17.0 / 17.9 ms
+// (before sincosf; 8 views forward + adjoint 28.9 / 28.8 / 29.0 / 29.4), builds with area
+// lights at 6 / 7 / 8 / 9 0.65 / 0.64 / 0.67 / 0.70 ms per Cornell frame.
 // k_shade sorts windows of kShadeWindow queue entries and shades them in rounds of 128.
 constexpr int kShadeRounds = 4, kShadeWindow = 128 * kShadeRounds;
+constexpr int kShadeBlocksEnv = 8, kShadeBlocksArea = 7;
 
 // Shading class of queue entry i: 0 a miss; else the hit material (light, Lambert, mirror,
 // dielectric, Phong, GGX) and, with kShadeSide, the side of the surface the ray arrives
@@ -699,8 +709,21 @@ __device__ __forceinline__ void shade_order(const WaveArgs& a, int p, int base, 
     __syncthreads();
 }
 
+// a ray of the any-hit queue (see k_shadow)
+__device__ __forceinline__ void put_shadow(const WaveArgs& a, bool have, int at, float3 o, float3 d, int dest, int job)
+{
+    if (!have) return;
+    if (at >= a.shadow_cap)
+    {
+        atomicOr(a.err, kErrQueue);
+        return;
+    }
+    __stcs(&a.so[0][at], make_float4(o.x, o.y, o.z, __int_as_float(dest)));
+    __stcs(&a.sd[0][at], make_float4(d.x, d.y, d.z, __int_as_float(job)));
+}
+
 template <bool ADJ, int LIGHTS = 3>
-__global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
+__global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlocksArea) k_shade(WaveArgs a, int p)
 {
     extern __shared__ float sgrad[];
     __shared__ int s_base[16], s_perm[kShadeWindow];
@@ -719,9 +742,13 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
         bool     cont = false;
         float3   phit = mk(0.f, 0.f, 0.f), cdir = mk(0.f, 0.f, 1.f), T2 = mk(0.f, 0.f, 0.f);
         float4   rnew = make_float4(0.f, 0.f, 0.f, 0.f);
-        int      flags2 = 0, n_nee = 0, job = 0, pixel = 0, nlog = 0;
-        uint64_t rstate = 0;
-        NeeRay   nee[4];
+        int      flags2 = 0, job = 0, pixel = 0, nlog = 0;
+        // a next-event vertex keeps what its rays are made from
+        bool             nee_here = false;
+        Mat              m;
+        float3           ns, wi, T;
+        VertexDraws      draws{0, 0};
+        const SceneView* scene = nullptr;
         unsigned lw[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
         if (valid)
         {
@@ -733,7 +760,8 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
             pixel = __float_as_int(d4.w);
             const JobGPU&    J = a.jobs[job];
             const SceneView& S = J.scene;
-            float3           T = xyz(t4);
+            scene = &S;
+            T = xyz(t4);
             const int        flags = __float_as_int(t4.w);
             const int        depth = (flags >> 8) & 0xff;
             bool             no_direct = depth == 0 || !(flags & 1);
@@ -761,8 +789,8 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
             else
             {
                 int    matid;
-                float3 ns = shading_normal(S, prim, hh.y, hh.z, matid);
-                Mat    m = load_mat(S, matid);
+                ns = shading_normal(S, prim, hh.y, hh.z, matid);
+                m = load_mat(S, matid);
                 if (m.consistent) ns = consistent_normal(S, prim, hh.y, hh.z, -d, ns);
                 phit = o + d * hh.x;
                 if (m.type == MAT_LGHT)
@@ -790,25 +818,16 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                         else
                             atomicOr(a.err, kErrQueue);
                     }
-                    Pcg rng;
-                    rng.state = a.qrng[p][i];
-                    rng.inc = (static_cast<uint64_t>(pixel) << 1u) | 1u;
-                    // the draws in a loop, not unrolled: smaller code (the kernel misses in
-                    // the instruction cache) and fewer spills; 24.9 -> 24.4 ms per cfg1 frame
-                    float u[NUM_DIMS];
-#pragma unroll 1
-                    for (int k = 0; k < NUM_DIMS; ++k) u[k] = rng.uniform();
-                    rstate = rng.state;
-                    float3 wi = -d;
-                    bool   nee_here = does_nee(m.type);
-                    if (nee_here) n_nee = make_nee<LIGHTS>(S, m, wi, ns, phit, T, u, nee);
-                    cont = continue_path(m, wi, ns, T, u, depth, J.max_depth, J.rr_depth, T2, cdir);
+                    draws.state = a.qrng[p][i];
+                    draws.inc = (static_cast<uint64_t>(pixel) << 1u) | 1u;
+                    wi = -d;
+                    nee_here = does_nee(m.type);
+                    cont = continue_path(m, wi, ns, T, draws, depth, J.max_depth, J.rr_depth, T2, cdir);
                     flags2 = (nee_here ? 1 : 0) | ((depth + 1) << 8) | (nlog << 20);
                 }
             }
             rnew = make_float4(rp.x + Ladd.x, rp.y + Ladd.y, rp.z + Ladd.z, rp.w);
         }
-        const int pend = (1 << n_nee) - 1;
         // continuing paths -> queue p ^ 1, ended paths -> finished list p ^ 1 (ballot + popc,
         // one atomic per warp each); dest: where this vertex's next-event results go
         int      dest = -1;
@@ -827,9 +846,8 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                     // leave the L2 to the tree (outdoor frame 84.6 -> 83.2 ms)
                     __stcs(&a.qo[pn][k], make_float4(phit.x, phit.y, phit.z, __int_as_float(job)));
                     __stcs(&a.qd[pn][k], make_float4(cdir.x, cdir.y, cdir.z, __int_as_float(pixel)));
-                    __stcs(&a.qthr[pn][k], make_float4(T2.x, T2.y, T2.z, __int_as_float(flags2 | (pend << 16))));
                     __stcs(&a.qrad[pn][k], rnew);
-                    __stcs(reinterpret_cast<unsigned long long*>(&a.qrng[pn][k]), static_cast<unsigned long long>(rstate));
+                    __stcs(reinterpret_cast<unsigned long long*>(&a.qrng[pn][k]), static_cast<unsigned long long>(draws.after()));
                     if (ADJ && nlog > 0)
                     {
                         a.qlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
@@ -855,7 +873,6 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                 if (k < a.capacity)
                 {
                     a.drad[pn][k] = rnew;
-                    a.dmeta[pn][k] = make_int4(pixel, job, pend, ADJ ? nlog : 0);
                     if (ADJ && nlog > 0)
                     {
                         a.dlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
@@ -869,41 +886,65 @@ __global__ void __launch_bounds__(128, 9) k_shade(WaveArgs a, int p)
                 }
             }
         }
-        if (dest < 0) n_nee = 0;  // no place for the results (queue overflow, reported)
-        // next-event rays: any-hit queue [0], closest-hit queue [1] (warp prefix sums)
-        int n_any = 0;
-        for (int r = 0; r < n_nee; ++r) n_any += nee[r].type == NEE_ENV ? 1 : 0;
-        int n_cl = n_nee - n_any;
-        for (int qsel = 0; qsel < 2; ++qsel)
+        // next-event rays: any-hit queue [0], closest-hit queue [1]; each is made, given a place
+        // in its queue and written before the next, so that none waits in local memory
+        if (dest < 0) nee_here = false;  // no place for the results (queue overflow, reported)
+        int pend = 0;
+        if ((LIGHTS & 1) && __any_sync(0xffffffffu, nee_here))
         {
-            int k = qsel == 0 ? n_any : n_cl;
-            int b = warp_append(&a.ctrl->scount[qsel], k);
-            int w = 0;
-            for (int r = 0; r < n_nee; ++r)
+            NeeRay r0, r1;
+            bool   h0 = false, h1 = false;
+            if (nee_here && scene->env_w > 0)
             {
-                if ((nee[r].type == NEE_ENV) != (qsel == 0)) continue;
-                int idx = b + w++;
-                if (idx >= a.shadow_cap)
+                h0 = nee_env_light(*scene, m, wi, ns, T, draws, r0);
+                if (h0) __stcs(&a.nev[pn][dest], r0.val);
+                h1 = nee_env_bsdf(*scene, m, wi, ns, T, draws, r1);
+                if (h1) __stcs(&a.nev[pn][dest + 1], r1.val);
+                pend = (h0 ? 1 : 0) | (h1 ? 2 : 0);
+            }
+            // a vertex's two rays side by side
+            const unsigned b0 = __ballot_sync(0xffffffffu, h0), b1 = __ballot_sync(0xffffffffu, h1);
+            int            base = 0;
+            if (lane == 0 && (b0 | b1)) base = atomicAdd(&a.ctrl->scount[0], __popc(b0) + __popc(b1));
+            base = __shfl_sync(0xffffffffu, base, 0) + __popc(b0 & lanemask_lt()) + __popc(b1 & lanemask_lt());
+            put_shadow(a, h0, base, phit, r0.d, dest, job);
+            put_shadow(a, h1, base + (h0 ? 1 : 0), phit, r1.d, dest + 1, job);
+        }
+        if ((LIGHTS & 2) && __any_sync(0xffffffffu, nee_here))
+        {
+            const bool area = nee_here && scene->light_area > 0.f;
+#pragma unroll
+            for (int which = 0; which < 2; ++which)
+            {
+                NeeRay r;
+                bool   h = false;
+                if (area)
+                    h = which == 0 ? nee_area_bsdf(*scene, m, wi, ns, phit, T, draws, r)
+                                   : nee_area_light(*scene, m, wi, ns, phit, T, draws, r);
+                const unsigned b = __ballot_sync(0xffffffffu, h);
+                if (!b) continue;
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&a.ctrl->scount[1], __popc(b));
+                base = __shfl_sync(0xffffffffu, base, 0) + __popc(b & lanemask_lt());
+                if (!h) continue;
+                pend |= 4 << which;
+                if (base >= a.shadow_cap)
                 {
                     atomicOr(a.err, kErrQueue);
-                    break;
+                    continue;
                 }
-                if (qsel == 0)
-                {
-                    __stcs(&a.so[0][idx], make_float4(phit.x, phit.y, phit.z, __int_as_float(dest + r)));
-                    __stcs(&a.sd[0][idx], make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, __int_as_float(job)));
-                    __stcs(&a.nev[pn][dest + r], nee[r].val);
-                }
-                else
-                {
-                    // .w: where a closest-hit ray stops at a nearer hit (tmin is kEpsRay for all)
-                    __stcs(&a.so[1][idx], make_float4(phit.x, phit.y, phit.z, nee[r].tterm));
-                    __stcs(&a.sd[1][idx], make_float4(nee[r].d.x, nee[r].d.y, nee[r].d.z, nee[r].tmax));
-                    a.sv[idx] = nee[r].val;
-                    a.sm[idx] = make_int4(dest + r, nee[r].type | (nee[r].light << 2), pixel, job);
-                }
+                // .w: where a closest-hit ray stops at a nearer hit (tmin is kEpsRay for all)
+                __stcs(&a.so[1][base], make_float4(phit.x, phit.y, phit.z, r.tterm));
+                __stcs(&a.sd[1][base], make_float4(r.d.x, r.d.y, r.d.z, r.tmax));
+                a.sv[base] = r.val;
+                a.sm[base] = make_int4(dest + 2 + which, r.type | (r.light << 2), pixel, job);
             }
         }
+        // the path's entry records which result slots will hold one
+        if (dest >= 0 && cont)
+            __stcs(&a.qthr[pn][dest >> 2], make_float4(T2.x, T2.y, T2.z, __int_as_float(flags2 | (pend << 16))));
+        else if (dest >= 0)
+            a.dmeta[pn][(dest >> 2) - a.capacity] = make_int4(pixel, job, pend, ADJ ? nlog : 0);
         pos += 128;
         if (pos % kShadeWindow == 0) pos += (gridDim.x - 1) * kShadeWindow;
     }
@@ -1127,7 +1168,7 @@ __global__ void __launch_bounds__(kPathBlock) k_paths(WaveArgs a, int64_t first,
             if (nee_here)
             {
                 NeeRay    nee[4];
-                const int nn = make_nee(S, m, wi, ns, phit, T, u, nee);
+                const int nn = make_nee(S, m, wi, ns, phit, T, ArrayDraws{u}, nee);
                 for (int r = 0; r < nn; ++r)
                 {
                     Hit        hs;
@@ -1145,7 +1186,7 @@ __global__ void __launch_bounds__(kPathBlock) k_paths(WaveArgs a, int64_t first,
                 }
             }
             float3     T2, cdir;
-            const bool cont = continue_path(m, wi, ns, T, u, depth, J.max_depth, J.rr_depth, T2, cdir);
+            const bool cont = continue_path(m, wi, ns, T, ArrayDraws{u}, depth, J.max_depth, J.rr_depth, T2, cdir);
             last_nee = nee_here;
             if (!cont) break;
             T = T2;
@@ -1300,7 +1341,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adjoint(AdjointArgs a)
             if (nee_here)
             {
                 NeeRay nee[4];
-                int    nn = make_nee(S, m, wi, ns, phit, T, u, nee);
+                int    nn = make_nee(S, m, wi, ns, phit, T, ArrayDraws{u}, nee);
                 for (int r = 0; r < nn; ++r)
                 {
                     Hit  hs;
@@ -1336,7 +1377,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adjoint(AdjointArgs a)
                 ++nlog;
             }
             float3 T2, cdir;
-            bool   cont = continue_path(m, wi, ns, T, u, depth, J.max_depth, J.rr_depth, T2, cdir);
+            bool   cont = continue_path(m, wi, ns, T, ArrayDraws{u}, depth, J.max_depth, J.rr_depth, T2, cdir);
             last_nee = nee_here;
             if (!cont) break;
             T = T2;
@@ -2046,6 +2087,20 @@ void enqueue_adjoint_iter(const WaveArgs& a, int p, const LaunchShape& ls, cudaS
     enqueue_iter<STACK, false, kTraceMinBlocks, true, REFM>(a, p, ls, st, nullptr);
 }
 
+// resident blocks per SM of the shading build for these lights
+template <bool ADJ>
+int shade_occupancy(int lights, size_t dynamic)
+{
+    int occ = 0;
+    if (lights == 1)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_shade<ADJ, 1>, 128, dynamic);
+    else if (lights == 2)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_shade<ADJ, 2>, 128, dynamic);
+    else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_shade<ADJ, 3>, 128, dynamic);
+    return std::max(occ, 1);
+}
+
 template <int STACK, bool REFM>
 int adjoint_launch_shape(const WaveArgs& a, LaunchShape& ls)
 {
@@ -2059,16 +2114,15 @@ int adjoint_launch_shape(const WaveArgs& a, LaunchShape& ls)
     constexpr int B = kTraceMinBlocks;
     CK(cudaFuncSetAttribute(k_connect<STACK, false, B, true, REFM>, cudaFuncAttributeMaxDynamicSharedMemorySize, dc));
     const int sms = num_sms();
-    int       occ_e = 0, occ_s = 0, occ_a = 0, occ_c = 0, occ_r = 0;
+    int       occ_e = 0, occ_a = 0, occ_c = 0, occ_r = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_e, k_extend<STACK, false, B, REFM>, kTraceBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_shade<true, 3>, 128, ds);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_regen<true>, 128, dr);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_shadow<STACK, false, B, REFM>, kTraceBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k_connect<STACK, false, B, true, REFM>, kTraceBlock, dc);
     ls.grid_trace = sms * std::max(occ_e, 1);
     ls.grid_any = sms * std::max(occ_a, 1);
     ls.grid_connect = sms * std::max(occ_c, 1);
-    ls.grid_shade = sms * std::max(occ_s, 1);
+    ls.grid_shade = sms * shade_occupancy<true>(ls.lights, ds);
     ls.grid_regen = sms * std::max(occ_r, 1);
     ls.grid_small = sms * 8;
     ls.block = 128;
@@ -2136,13 +2190,13 @@ int adjoint_stream(Workspace& w, const std::vector<JobGPU>& jobs, int64_t total,
         lights |= (J.scene.env_w > 0 ? 1 : 0) | (J.scene.light_area > 0.f ? 2 : 0);
     }
     LaunchShape ls;
+    ls.fast_only = fast_only;
+    ls.lights = lights == 0 ? 3 : lights;
     rc = stack32 ? (fast_only ? adjoint_launch_shape<kSmallStack, false>(a, ls)
                               : adjoint_launch_shape<kSmallStack, true>(a, ls))
                  : (fast_only ? adjoint_launch_shape<kStack, false>(a, ls)
                               : adjoint_launch_shape<kStack, true>(a, ls));
     if (rc) return rc;
-    ls.fast_only = fast_only;
-    ls.lights = lights == 0 ? 3 : lights;
     run.iter_launches = 4 + (ls.lights & 1) + (ls.lights >> 1);
     auto iter = [&](cudaStream_t s2, int p, StageTimer*) {
         if (stack32)
@@ -2242,8 +2296,7 @@ int render_jobs(int num_jobs, mcrt_scene* const* scenes, const mcrt_camera* cams
         fast_only = fast_only && J.traverse != MCRT_TRAVERSE_REF;
         lights |= (J.scene.env_w > 0 ? 1 : 0) | (J.scene.light_area > 0.f ? 2 : 0);
     }
-    LaunchShape lsv = launch_shape_variant(stack32, regcap, fast_only);
-    lsv.lights = lights == 0 ? 3 : lights;
+    LaunchShape lsv = launch_shape_variant(stack32, regcap, fast_only, lights == 0 ? 3 : lights);
     Workspace&  w = dw.ws;
     w.args.batch_fetch = (vb & MCRT_VARIANT_GRIDSTRIDE) ? 0 : 1;
     StageTimer  timer;
@@ -2380,11 +2433,11 @@ void traversal_occupancy(int& extend, int& shadow, int& connect)
 }
 }  // namespace
 
-LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only)
+LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only, int lights)
 {
     LaunchShape   ls;
     const int     sms = num_sms();
-    int           occ_t = 0, occ_a = 0, occ_c = 0, occ_s = 0;
+    int           occ_t = 0, occ_a = 0, occ_c = 0, occ_r = 0;
     constexpr int B = kTraceMinBlocks;
     if (!fast_only)  // the general build (see with_variant)
         traversal_occupancy<kStack, 1, true>(occ_t, occ_a, occ_c);
@@ -2395,12 +2448,13 @@ LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only)
         regcap ? traversal_occupancy<kStack, B, false>(occ_t, occ_a, occ_c)
                : traversal_occupancy<kStack, 1, false>(occ_t, occ_a, occ_c);
     ls.fast_only = fast_only;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_shade<false>, 128, 0);
+    ls.lights = lights;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_regen<false>, 128, 0);
     ls.grid_trace = sms * std::max(occ_t, 1);
     ls.grid_any = sms * std::max(occ_a, 1);
     ls.grid_connect = sms * std::max(occ_c, 1);
-    ls.grid_shade = sms * std::max(occ_s, 1);
-    ls.grid_regen = ls.grid_shade;
+    ls.grid_shade = sms * shade_occupancy<false>(lights, 0);
+    ls.grid_regen = sms * std::max(occ_r, 1);
     ls.grid_small = sms * 8;
     ls.block = 128;
     return ls;

@@ -160,7 +160,7 @@ int64_t stream_ring_entries(int64_t capacity, int max_depth, int64_t max_spp, in
 int wave_iterations(int max_depth);
 // persistent grid sizes from the SM count and occupancy (queries only, no allocation)
 LaunchShape launch_shape();
-LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only = false);
+LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only = false, int lights = 3);
 // starts a render: zeroes the counters and sets the admission limit (`limit`; with `waves`
 // nothing is admitted until the first wave's k_wave_next) -- one kernel, so it may run
 // inside a stream capture; the per-pixel counts of the ring must be zero
