@@ -4,9 +4,8 @@
 //   k_trace<ANY, MODE, STACK, MINB>  batch closest/any-hit queries (SceneBVH::intersect / occluded)
 //   wavefront iterations (wavefront.h; all graph-capturable: every count is read from
 //   device memory, grids are fixed):
-//     k_render_begin, k_wave_next, k_iter_begin   counters and admission
-//     k_regen            finish ended paths (ring, in-order pixel resolve) and start
-//                        camera paths with the tent filter (demo_pt.cpp:689-708)
+//     k_render_begin, k_wave_next, k_admit   counters and admission
+//     k_start            camera paths with the tent filter (demo_pt.cpp:689-708)
 //     k_extend           closest hit of the ray queue
 //     k_shade            one vertex of rayTrace (demo_pt.cpp:523-651): emission, NEE with
 //                        MIS against the environment and the area lights, continuation,
@@ -17,6 +16,7 @@
 //     k_shadow           next-event rays to the environment: any hit
 //     k_connect          next-event rays to area lights: bounded closest hit (which must be
 //                        the sampled emitter), MIS-weighted
+//     k_finish           ended paths: ring, in-order pixel resolve
 //   k_adjoint            path-replay adjoint (one thread per path, replayed from its seed)
 #include <cuda_runtime.h>
 
@@ -193,44 +193,12 @@ __device__ __forceinline__ float4 add_pending(const float4* slots, int mask, flo
     return r;
 }
 
-// counters of a new render; the wave schedule admits nothing until k_wave_next
-__global__ void k_render_begin(WaveArgs a, int waves, int64_t limit)
+// tops queue p up with new paths (continuing rays are already in it)
+__device__ __forceinline__ void admit(Ctrl* c, int64_t capacity, int p)
 {
-    Ctrl* c = a.ctrl;
-    c->qcount[0] = c->qcount[1] = 0;
-    c->dcount[0] = c->dcount[1] = 0;
-    c->scount[0] = c->scount[1] = 0;
-    c->new_base = c->new_count = 0;
-    c->chunk = -1;
-    c->fetch[0] = c->fetch[1] = c->fetch[2] = 0;
-    c->next = 0;
-    c->limit = waves ? 0ull : static_cast<unsigned long long>(limit);
-    c->new_g = 0;
-    c->finished = 0;
-}
-
-// wave schedule: admit the next wave's paths
-__global__ void k_wave_next(WaveArgs a)
-{
-    Ctrl* c = a.ctrl;
-    c->chunk += 1;
-    c->limit = static_cast<unsigned long long>(a.chunk_table[c->chunk + 1]);
-}
-
-__global__ void k_iter_begin(WaveArgs a, int p)
-{
-    Ctrl* c = a.ctrl;
-    c->qcount[p ^ 1] = 0;
-    c->dcount[p ^ 1] = 0;
-    c->scount[0] = 0;
-    c->scount[1] = 0;
-    c->fetch[0] = 0;
-    c->fetch[1] = 0;
-    c->fetch[2] = 0;
-    // top the queue up with new paths (continuing rays are already in it)
     const int                q = c->qcount[p];
     const unsigned long long avail = c->limit > c->next ? c->limit - c->next : 0ull;
-    const long long          room = a.capacity - static_cast<long long>(q);
+    const long long          room = capacity - static_cast<long long>(q);
     const int n = room > 0 ? static_cast<int>(avail < static_cast<unsigned long long>(room) ? avail : room) : 0;
     c->new_base = q;
     c->new_count = n;
@@ -239,15 +207,43 @@ __global__ void k_iter_begin(WaveArgs a, int p)
     c->next += static_cast<unsigned long long>(n);
 }
 
+// counters of a new render; the wave schedule admits nothing until k_wave_next
+__global__ void k_render_begin(WaveArgs a, int waves, int64_t limit)
+{
+    Ctrl* c = a.ctrl;
+    for (int p = 0; p < 2; ++p)
+    {
+        c->qcount[p] = c->dcount[p] = 0;
+        c->scount[p][0] = c->scount[p][1] = 0;
+        c->fetch[p][0] = c->fetch[p][1] = c->fetch[p][2] = 0;
+    }
+    c->chunk = -1;
+    c->next = 0;
+    c->limit = waves ? 0ull : static_cast<unsigned long long>(limit);
+    c->finished = 0;
+    admit(c, a.capacity, 0);
+}
+
+// wave schedule: admit the next wave's paths (parity 0: a wave has an even number of iterations)
+__global__ void k_wave_next(WaveArgs a)
+{
+    Ctrl* c = a.ctrl;
+    c->chunk += 1;
+    c->limit = static_cast<unsigned long long>(a.chunk_table[c->chunk + 1]);
+    admit(c, a.capacity, 0);
+}
+
+__global__ void k_admit(WaveArgs a, int p) { admit(a.ctrl, a.capacity, p); }
+
 // Gradient accumulators of an adjoint launch.  A kernel adds to the albedo gradients
-// (GRAD_ALBEDO: k_regen, k_shade), to the emission gradients (GRAD_EMISSION: k_shade,
+// (GRAD_ALBEDO: k_finish, k_shade), to the emission gradients (GRAD_EMISSION: k_shade,
 // k_connect) or both; each part it adds to is kept per block in shared memory when
 // WaveArgs::grad_shared has that part's bit (flushed with one global atomic per nonzero
 // entry when the block ends), and goes straight to the global vector otherwise.  A kernel's
 // dynamic shared memory is the parts it uses (grad_smem_bytes), so the next-event kernels
 // hold no albedo slice and keep their occupancy when there are thousands of albedos.
 constexpr int GRAD_ALBEDO = 1, GRAD_EMISSION = 2;
-// A part is kept per block while it fits 20 KB: then k_shade and k_regen keep their 9
+// A part is kept per block while it fits 20 KB: then k_shade and k_finish keep their
 // blocks per SM.  Few parameters need it (global atomics on cfg3's 256 albedos: adjoint
 // 127 ms instead of 11.8); many do better in global memory at full occupancy (cfg4's 4096
 // albedos, 48 KB: forward + adjoint 106.9 ms in global memory, 113.4 per block).
@@ -480,26 +476,27 @@ __device__ __forceinline__ void finish_paths(const WaveArgs& a, const Grads& G, 
     }
 }
 
+__global__ void __launch_bounds__(128) k_start(WaveArgs a, int p)
+{
+    const Ctrl*   c = a.ctrl;
+    const int     n = c->new_count, base = c->new_base;
+    const int64_t g0 = static_cast<int64_t>(c->new_g);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        start_camera_path(a, g0 + i, p, base + i);
+}
+
+// finished list p
 template <bool ADJ>
-__global__ void __launch_bounds__(128) k_regen(WaveArgs a, int p)
+__global__ void __launch_bounds__(128) k_finish(WaveArgs a, int p)
 {
     extern __shared__ float sgrad[];
     const Grads        G = grads_begin<ADJ, GRAD_ALBEDO>(a, sgrad);
-    const Ctrl*        c = a.ctrl;
-    const int          nd = min(c->dcount[p], static_cast<int>(a.capacity));
-    const int          nn = c->new_count;
-    const int          nb = c->new_base;
-    const int64_t      g0 = static_cast<int64_t>(c->new_g);
-    const int          n = max(nd, nn);
+    const int          n = min(a.ctrl->dcount[p], static_cast<int>(a.capacity));
     const int          lane = threadIdx.x & 31;
     const int          warps_total = (gridDim.x * blockDim.x) >> 5;
     unsigned long long fin = 0;
     for (int wbase = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; wbase < n; wbase += warps_total * 32)
-    {
-        const int i = wbase + lane;
-        if (wbase < nd) finish_paths<ADJ>(a, G, p, i, i < nd, fin);
-        if (i < nn) start_camera_path(a, g0 + i, p, nb + i);
-    }
+        finish_paths<ADJ>(a, G, p, wbase + lane, wbase + lane < n, fin);
     for (int off = 16; off > 0; off >>= 1) fin += __shfl_down_sync(0xffffffffu, fin, off);
     if (lane == 0 && fin) atomicAdd(&a.ctrl->finished, fin);
     grads_end<ADJ, GRAD_ALBEDO>(a, sgrad);
@@ -570,7 +567,7 @@ struct ExtendRays : QueueFetch
     const WaveArgs& a;
     int             p;
     __device__ __forceinline__ ExtendRays(const WaveArgs& a_, int p_)
-        : QueueFetch(&a_.ctrl->fetch[0], a_.batch_fetch != 0), a(a_), p(p_)
+        : QueueFetch(&a_.ctrl->fetch[p_][0], a_.batch_fetch != 0), a(a_), p(p_)
     {
     }
     __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.qo[p][i] : &a.qd[p][i]; }
@@ -599,7 +596,12 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
 {
     const int  n = min(a.ctrl->qcount[p], static_cast<int>(a.capacity));
     TraceCount cnt = {0u, 0u};
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats[0], static_cast<unsigned long long>(n));
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        atomicAdd(&a.stats[0], static_cast<unsigned long long>(n));
+        a.ctrl->qcount[p ^ 1] = 0;  // (see Ctrl)
+        a.ctrl->dcount[p ^ 1] = 0;
+    }
     if constexpr (!REFM && kStreamTraversal)
     {
         __shared__ StreamSmem<STACK, kTraceBlock> sm;
@@ -611,7 +613,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
         __shared__ int stack[STACK * kTraceBlock];
         int*           st = stack + threadIdx.x;
         const float    inf = __int_as_float(0x7f800000);
-        for (QueueWalk w(&a.ctrl->fetch[0], n, a.batch_fetch != 0); w.valid(); w.next())
+        for (QueueWalk w(&a.ctrl->fetch[p][0], n, a.batch_fetch != 0); w.valid(); w.next())
         {
             const int i = w.i;
             if (i >= n) continue;
@@ -731,6 +733,11 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
     const int n = min(a.ctrl->qcount[p], static_cast<int>(a.capacity));
     const int lane = threadIdx.x & 31;
     const int pn = p ^ 1;
+    if (blockIdx.x == 0 && threadIdx.x < 3)  // (see Ctrl)
+    {
+        a.ctrl->fetch[pn][threadIdx.x] = 0;
+        if (threadIdx.x < 2) a.ctrl->scount[pn][threadIdx.x] = 0;
+    }
     // pos: the first entry of this round; windows start at multiples of kShadeWindow, and a
     // window's valid entries fill its first rounds (the sort puts entries past n last)
     for (int pos = blockIdx.x * kShadeWindow; pos < n;)  // blocks of 128 threads
@@ -905,7 +912,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
             // a vertex's two rays side by side
             const unsigned b0 = __ballot_sync(0xffffffffu, h0), b1 = __ballot_sync(0xffffffffu, h1);
             int            base = 0;
-            if (lane == 0 && (b0 | b1)) base = atomicAdd(&a.ctrl->scount[0], __popc(b0) + __popc(b1));
+            if (lane == 0 && (b0 | b1)) base = atomicAdd(&a.ctrl->scount[p][0], __popc(b0) + __popc(b1));
             base = __shfl_sync(0xffffffffu, base, 0) + __popc(b0 & lanemask_lt()) + __popc(b1 & lanemask_lt());
             put_shadow(a, h0, base, phit, r0.d, dest, job);
             put_shadow(a, h1, base + (h0 ? 1 : 0), phit, r1.d, dest + 1, job);
@@ -924,7 +931,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                 const unsigned b = __ballot_sync(0xffffffffu, h);
                 if (!b) continue;
                 int base = 0;
-                if (lane == 0) base = atomicAdd(&a.ctrl->scount[1], __popc(b));
+                if (lane == 0) base = atomicAdd(&a.ctrl->scount[p][1], __popc(b));
                 base = __shfl_sync(0xffffffffu, base, 0) + __popc(b & lanemask_lt());
                 if (!h) continue;
                 pend |= 4 << which;
@@ -983,7 +990,7 @@ struct ShadowRays : QueueFetch
     const WaveArgs& a;
     int             p;
     __device__ __forceinline__ ShadowRays(const WaveArgs& a_, int p_)
-        : QueueFetch(&a_.ctrl->fetch[1], a_.batch_fetch != 0), a(a_), p(p_)
+        : QueueFetch(&a_.ctrl->fetch[p_][1], a_.batch_fetch != 0), a(a_), p(p_)
     {
     }
     __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.so[0][i] : &a.sd[0][i]; }
@@ -1007,7 +1014,7 @@ template <int STACK, bool COUNT, int MINB, bool REFM = true>
 __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kAnyHitMinBlocks : MINB) k_shadow(WaveArgs a, int p)
 {
     TraceCount cnt = {0u, 0u};
-    const int  n = min(a.ctrl->scount[0], static_cast<int>(a.shadow_cap));
+    const int  n = min(a.ctrl->scount[p][0], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
     if constexpr (!REFM && kStreamTraversal)
     {
@@ -1019,7 +1026,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kAnyHitMinBlocks : MIN
     {
         __shared__ int stack[STACK * kTraceBlock];
         int*           st = stack + threadIdx.x;
-        for (QueueWalk w(&a.ctrl->fetch[1], n, a.batch_fetch != 0); w.valid(); w.next())
+        for (QueueWalk w(&a.ctrl->fetch[p][1], n, a.batch_fetch != 0); w.valid(); w.next())
         {
             const int k = w.i;
             if (k >= n) continue;
@@ -1042,7 +1049,7 @@ struct ConnectRays : QueueFetch
     const Grads&    G;
     int             p;
     __device__ __forceinline__ ConnectRays(const WaveArgs& a_, const Grads& G_, int p_)
-        : QueueFetch(&a_.ctrl->fetch[2], a_.batch_fetch != 0), a(a_), G(G_), p(p_)
+        : QueueFetch(&a_.ctrl->fetch[p_][2], a_.batch_fetch != 0), a(a_), G(G_), p(p_)
     {
     }
     __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.so[1][i] : &a.sd[1][i]; }
@@ -1074,7 +1081,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kConnectMinBlocks : MI
     extern __shared__ float sgrad[];
     const Grads             G = grads_begin<ADJ, GRAD_EMISSION>(a, sgrad);
     TraceCount              cnt = {0u, 0u};
-    const int               n = min(a.ctrl->scount[1], static_cast<int>(a.shadow_cap));
+    const int               n = min(a.ctrl->scount[p][1], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
     if constexpr (!REFM && kStreamTraversal)
     {
@@ -1086,7 +1093,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kConnectMinBlocks : MI
     {
         __shared__ int stack[STACK * kTraceBlock];
         int*           st = stack + threadIdx.x;
-        for (QueueWalk w(&a.ctrl->fetch[2], n, a.batch_fetch != 0); w.valid(); w.next())
+        for (QueueWalk w(&a.ctrl->fetch[p][2], n, a.batch_fetch != 0); w.valid(); w.next())
         {
             const int k = w.i;
             if (k >= n) continue;
@@ -1441,6 +1448,17 @@ int fail(int code, const std::string& msg)
                         std::string(#x) + ": " + cudaGetErrorString(e_));                         \
     } while (0)
 
+// Where an iteration's kernels go: k_shadow, k_connect and k_finish to `side`, beside the next
+// iteration's k_extend on `main`; `fork` / `join` order them after this k_shade and before the
+// next.  side == main: one after another, no events.  Small launches overlap their ramps and
+// tails (a 61x47 preview 0.69 -> 0.56 ms, a Cornell frame of 1 M paths 2.09 -> 1.87, 12 mixed
+// scenes 17.0 -> 16.1), a full queue gains a little (outdoor frame 80.4 -> 78.1 ms).
+struct IterStreams
+{
+    cudaStream_t main, side;
+    cudaEvent_t  fork, join;
+};
+
 struct Workspace
 {
     int64_t             capacity = 0;  // rays per queue of `block`
@@ -1456,6 +1474,8 @@ struct Workspace
     unsigned long long* stats = nullptr;
     int*                err = nullptr;
     unsigned long long* h_poll = nullptr;  // pinned: completion polls of the streaming schedule
+    cudaStream_t        side = nullptr;    // IterStreams
+    cudaEvent_t         fork = nullptr, join = nullptr;
     int64_t             adj_capacity = 0;    // rays per queue of `adj_block`
     void*               adj_block = nullptr; // adjoint vertex logs
 };
@@ -1634,6 +1654,9 @@ int ensure_workspace(Workspace& w, int64_t capacity, int64_t ring, int num_jobs,
         CK(cudaMalloc(&w.stats, sizeof(unsigned long long) * 8));
         CK(cudaMalloc(&w.err, sizeof(int)));
         CK(cudaMallocHost(&w.h_poll, 2 * sizeof(unsigned long long)));
+        CK(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
     }
     if (w.block) carve_queues(w.args, w.block, w.capacity);
     if (w.ring_block) carve_ring(w.args, w.ring_block, w.ring);
@@ -1672,41 +1695,49 @@ struct StageTimer
     }
 };
 
-// one iteration of parity p (six launches); stage timer slots: 0 begin + regen,
-// 1 extend, 2 shade, 3 connect
+// one iteration of parity p; stage timer slots: 0 admission, start and finish, 1 extend,
+// 2 shade, 3 next-event rays (a timed iteration runs on one stream).  after_side: the
+// iteration before left work on the side stream.
 template <int STACK, bool COUNT, int MINB, bool ADJ = false, bool REFM = true>
-void enqueue_iter(const WaveArgs& a, int p, const LaunchShape& ls, cudaStream_t st, StageTimer* tm)
+void enqueue_iter(const WaveArgs& a, int p, const LaunchShape& ls, const IterStreams& s, bool after_side, StageTimer* tm)
 {
     // adjoint: each kernel's shared gradient slices (0 for the forward)
     const size_t dr = ADJ ? grad_smem_bytes(a, GRAD_ALBEDO) : 0;
     const size_t ds = ADJ ? grad_smem_bytes(a, GRAD_ALBEDO | GRAD_EMISSION) : 0;
     const size_t dc = ADJ ? grad_smem_bytes(a, GRAD_EMISSION) : 0;
+    const bool   split = s.side != s.main;
     auto beg = [&](int stg) {
-        if (tm) tm->record(st, stg, true);
+        if (tm) tm->record(s.main, stg, true);
     };
     auto end = [&]() {
-        if (tm) tm->record(st, 0, false);
+        if (tm) tm->record(s.main, 0, false);
     };
-    beg(0);
-    k_iter_begin<<<1, 1, 0, st>>>(a, p);
-    k_regen<ADJ><<<ls.grid_regen, 128, dr, st>>>(a, p);
-    end();
     beg(1);
-    k_extend<STACK, COUNT, MINB, REFM><<<ls.grid_trace, kTraceBlock, 0, st>>>(a, p);
+    k_extend<STACK, COUNT, MINB, REFM><<<ls.grid_trace, kTraceBlock, 0, s.main>>>(a, p);
     end();
+    if (split && after_side) cudaStreamWaitEvent(s.main, s.join, 0);
     beg(2);
     if (ls.lights == 1)
-        k_shade<ADJ, 1><<<ls.grid_shade, 128, ds, st>>>(a, p);
+        k_shade<ADJ, 1><<<ls.grid_shade, 128, ds, s.main>>>(a, p);
     else if (ls.lights == 2)
-        k_shade<ADJ, 2><<<ls.grid_shade, 128, ds, st>>>(a, p);
+        k_shade<ADJ, 2><<<ls.grid_shade, 128, ds, s.main>>>(a, p);
     else
-        k_shade<ADJ, 3><<<ls.grid_shade, 128, ds, st>>>(a, p);
+        k_shade<ADJ, 3><<<ls.grid_shade, 128, ds, s.main>>>(a, p);
     end();
+    if (split)
+    {
+        cudaEventRecord(s.fork, s.main);
+        cudaStreamWaitEvent(s.side, s.fork, 0);
+    }
     beg(3);
     // each kind of next-event ray exists only where a job has that kind of light
-    if (ls.lights & 1) k_shadow<STACK, COUNT, MINB, REFM><<<ls.grid_any, kTraceBlock, 0, st>>>(a, p);
-    if (ls.lights & 2) k_connect<STACK, COUNT, MINB, ADJ, REFM><<<ls.grid_connect, kTraceBlock, dc, st>>>(a, p);
+    if (ls.lights & 1) k_shadow<STACK, COUNT, MINB, REFM><<<ls.grid_any, kTraceBlock, 0, s.side>>>(a, p);
+    if (ls.lights & 2) k_connect<STACK, COUNT, MINB, ADJ, REFM><<<ls.grid_connect, kTraceBlock, dc, s.side>>>(a, p);
     end();
+    beg(0);
+    k_finish<ADJ><<<ls.grid_regen, 128, dr, s.side>>>(a, p ^ 1);
+    end();
+    if (split) cudaEventRecord(s.join, s.side);
 }
 
 // one wave of the wave schedule: admit the wave, then iterate until its last path is
@@ -1716,9 +1747,11 @@ void enqueue_wave(const WaveArgs& a, int max_depth, const LaunchShape& ls, cudaS
 {
     if (tm) tm->record(st, 0, true);
     k_wave_next<<<1, 1, 0, st>>>(a);
+    k_start<<<ls.grid_regen, 128, 0, st>>>(a, 0);
     if (tm) tm->record(st, 0, false);
-    const int iters = wave_iterations(max_depth);
-    for (int t = 0; t < iters; ++t) enqueue_iter<STACK, COUNT, MINB, false, REFM>(a, t & 1, ls, st, tm);
+    const int         iters = wave_iterations(max_depth);
+    const IterStreams s{st, st, nullptr, nullptr};
+    for (int t = 0; t < iters; ++t) enqueue_iter<STACK, COUNT, MINB, false, REFM>(a, t & 1, ls, s, false, tm);
 }
 
 int validate_job_impl(const mcrt_scene* s, const mcrt_camera* c, const mcrt_render_params* p)
@@ -1747,7 +1780,7 @@ struct RunResult
     int64_t     launches = 0;
     int64_t     extend_launches = 0;
     int64_t     table_bytes = 0;  // host -> device besides the job table
-    int         iter_launches = 6;  // launches per iteration (5 with one kind of light)
+    int         iter_launches = 5;  // launches per iteration (4 with one kind of light)
     int64_t     poll_bytes = 0;   // device -> host completion polls
 };
 
@@ -1770,12 +1803,13 @@ struct IterEnqueue
     const WaveArgs*    a;
     int                p;
     const LaunchShape* ls;
-    cudaStream_t       st;
+    const IterStreams* s;
+    bool               after_side;
     StageTimer*        tm;
     template <int S, bool C, int M, bool R>
     void run() const
     {
-        enqueue_iter<S, C, M, false, R>(*a, p, *ls, st, tm);
+        enqueue_iter<S, C, M, false, R>(*a, p, *ls, *s, after_side, tm);
     }
 };
 
@@ -1882,7 +1916,7 @@ int run_waves(Workspace& w, const std::vector<JobGPU>& jobs, const std::vector<i
     run.table_bytes = 8 * static_cast<int64_t>(table.size());
     const int iters = wave_iterations(max_depth);
     run.waves = num_chunks;
-    run.launches = 1 + num_chunks * (1 + run.iter_launches * iters);
+    run.launches = 1 + num_chunks * (2 + run.iter_launches * iters);
     run.extend_launches = num_chunks * iters;
     auto enqueue = [&](cudaStream_t s2, StageTimer* tm) {
         with_variant(stack32, regcap, count, WaveEnqueue{&a, max_depth, &lsv, s2, tm});
@@ -1955,21 +1989,39 @@ int run_paths(Workspace& w, const std::vector<JobGPU>& jobs, const std::vector<i
     return MCRT_OK;
 }
 
-// Iterations in graph-launched pairs (parity 0, 1) until every path is finished, which
-// the host learns from a device counter polled one batch behind the launches.
-// iter(stream, parity, timer) enqueues one iteration.
+// Iterations (parity 0, 1 in turn) until every path is finished.  Paths that all fit the queue
+// are admitted at once and need max_depth + 1 iterations; otherwise each iteration tops the
+// queue up first.  The host learns from a device counter, copied after each pair of iterations
+// and read one pair behind the launches, when no path is left (before, it was read every eight
+// iterations: a 61x47 frame of depth 4 ran 16 iterations instead of 5).
+// iter(streams, parity, after_side, timer) enqueues one iteration.
 template <class IterFn>
-int stream_loop(Workspace& w, const WaveArgs& a, int64_t total, int max_depth, bool stages, bool graph,
-                cudaStream_t st, StageTimer& timer, RunResult& run, const IterFn& iter)
+int stream_loop(Workspace& w, const WaveArgs& a, const LaunchShape& ls, int64_t total, int max_depth, bool stages,
+                bool graph, cudaStream_t st, StageTimer& timer, RunResult& run, const IterFn& iter)
 {
     // while paths remain to be admitted every iteration traces a full queue, each path
     // has at most max_depth + 1 rays in queues, and a path is finished at most
-    // max_depth + 2 iterations after admission
-    const int64_t bound = (total * (max_depth + 1) + a.capacity - 1) / a.capacity + max_depth + 2;
-    constexpr int kPairsPerPoll = 4;
+    // max_depth + 1 iterations after admission
+    const bool    at_once = total <= a.capacity;
+    const int64_t bound = at_once ? max_depth + 1
+                                  : (total * (max_depth + 1) + a.capacity - 1) / a.capacity + max_depth + 1;
+    const IterStreams s{st, stages ? st : w.side, w.fork, w.join};
     CK(cudaEventRecord(run.e0, st));
     k_render_begin<<<1, 1, 0, st>>>(a, 0, total);
-    run.launches = 1;
+    k_start<<<ls.grid_regen, 128, 0, st>>>(a, 0);
+    run.launches = 2;
+    // one iteration, after the first with an admission before it where paths are left to admit
+    // (with nothing left it starts none)
+    auto one = [&](const IterStreams& is, int p, bool first, bool after_side, StageTimer* tm) {
+        if (!at_once && !first)
+        {
+            if (tm) tm->record(is.main, 0, true);
+            k_admit<<<1, 1, 0, is.main>>>(a, p);
+            k_start<<<ls.grid_regen, 128, 0, is.main>>>(a, p);
+            if (tm) tm->record(is.main, 0, false);
+        }
+        iter(is, p, after_side, tm);
+    };
     cudaGraph_t     g = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t    cap = nullptr;
@@ -1982,9 +2034,11 @@ int stream_loop(Workspace& w, const WaveArgs& a, int64_t total, int max_depth, b
     {
         CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        iter(cap, 0, nullptr);
-        iter(cap, 1, nullptr);
-        cudaError_t e = cudaStreamEndCapture(cap, &g);
+        const IterStreams c{cap, w.side, w.fork, w.join};
+        one(c, 0, false, false, nullptr);
+        one(c, 1, false, true, nullptr);
+        cudaError_t e = cudaStreamWaitEvent(cap, w.join, 0);
+        if (e == cudaSuccess) e = cudaStreamEndCapture(cap, &g);
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
         if (e != cudaSuccess)
         {
@@ -1995,36 +2049,36 @@ int stream_loop(Workspace& w, const WaveArgs& a, int64_t total, int max_depth, b
     cudaEvent_t poll_ev[2] = {nullptr, nullptr};
     cudaError_t e = cudaEventCreateWithFlags(&poll_ev[0], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&poll_ev[1], cudaEventDisableTiming);
-    int64_t iters = 0;
-    bool    done = false;
+    int64_t            iters = 0;
+    bool               done = false;
+    const cudaStream_t last = graph ? st : s.side;  // where a pair's k_finish is
     for (int b = 0; !done && e == cudaSuccess; ++b)
     {
-        for (int k = 0; k < kPairsPerPoll && e == cudaSuccess; ++k)
+        if (graph)
         {
-            if (graph)
-            {
-                e = cudaGraphLaunch(exec, st);
-            }
-            else
-            {
-                iter(st, 0, stages ? &timer : nullptr);
-                iter(st, 1, stages ? &timer : nullptr);
-                e = cudaGetLastError();
-            }
+            e = cudaGraphLaunch(exec, st);
             iters += 2;
         }
-        if (e != cudaSuccess) break;
-        e = cudaMemcpyAsync(&w.h_poll[b & 1], &a.ctrl->finished, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                            st);
-        if (e == cudaSuccess) e = cudaEventRecord(poll_ev[b & 1], st);
+        else
+        {
+            for (int k = 0; k < 2 && !(at_once && iters >= bound); ++k, ++iters)
+                one(s, k, iters == 0, iters > 0, stages ? &timer : nullptr);
+            e = cudaGetLastError();
+        }
+        if (at_once && iters >= bound) break;
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&w.h_poll[b & 1], &a.ctrl->finished, sizeof(unsigned long long),
+                                cudaMemcpyDeviceToHost, last);
+        if (e == cudaSuccess) e = cudaEventRecord(poll_ev[b & 1], last);
         run.poll_bytes += sizeof(unsigned long long);
         if (e == cudaSuccess && b >= 1)
         {
             e = cudaEventSynchronize(poll_ev[(b - 1) & 1]);
             if (e == cudaSuccess && static_cast<int64_t>(w.h_poll[(b - 1) & 1]) >= total) done = true;
         }
-        if (e == cudaSuccess && !done && iters > bound + 4 * kPairsPerPoll)
+        if (e == cudaSuccess && !done && iters > bound + 8)
         {
+            cudaStreamSynchronize(s.side);
             cudaStreamSynchronize(st);
             cudaEventDestroy(poll_ev[0]);
             cudaEventDestroy(poll_ev[1]);
@@ -2032,14 +2086,19 @@ int stream_loop(Workspace& w, const WaveArgs& a, int64_t total, int max_depth, b
             return fail(MCRT_ERR_INTERNAL, "streaming render did not finish within its iteration bound");
         }
     }
+    if (e == cudaSuccess && !graph && s.side != st) e = cudaStreamWaitEvent(st, w.join, 0);
     if (e == cudaSuccess) e = cudaEventRecord(run.e1, st);
     if (e == cudaSuccess && graph) e = cudaStreamSynchronize(st);  // before the graph is destroyed
     if (poll_ev[0]) cudaEventDestroy(poll_ev[0]);
     if (poll_ev[1]) cudaEventDestroy(poll_ev[1]);
     release_graph();
-    if (e != cudaSuccess) return fail(MCRT_ERR_CUDA, std::string("streaming render: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess)
+    {
+        cudaStreamSynchronize(s.side);
+        return fail(MCRT_ERR_CUDA, std::string("streaming render: ") + cudaGetErrorString(e));
+    }
     run.waves = iters;
-    run.launches += iters * run.iter_launches;
+    run.launches += iters * run.iter_launches + (at_once ? 0 : 2 * (graph ? iters : iters - 1));
     run.extend_launches = iters;
     return MCRT_OK;
 }
@@ -2070,10 +2129,10 @@ int run_stream(Workspace& w, const std::vector<JobGPU>& jobs, const std::vector<
         break;
     }
     if (rc) return rc;
-    auto iter = [&](cudaStream_t s2, int p, StageTimer* tm) {
-        with_variant(stack32, regcap, count, IterEnqueue{&a, p, &lsv, s2, tm});
+    auto iter = [&](const IterStreams& s, int p, bool after_side, StageTimer* tm) {
+        with_variant(stack32, regcap, count, IterEnqueue{&a, p, &lsv, &s, after_side, tm});
     };
-    return stream_loop(w, a, total, max_depth, stages, graph, st, timer, run, iter);
+    return stream_loop(w, a, lsv, total, max_depth, stages, graph, st, timer, run, iter);
 }
 
 // Path-replay adjoint on the streaming wavefront: the forward's stages with ADJ set (see
@@ -2082,9 +2141,9 @@ int run_stream(Workspace& w, const std::vector<JobGPU>& jobs, const std::vector<
 // REFM = false when every job traverses in FAST mode; the shading build follows ls.lights
 // (the forward's specialisations)
 template <int STACK, bool REFM>
-void enqueue_adjoint_iter(const WaveArgs& a, int p, const LaunchShape& ls, cudaStream_t st)
+void enqueue_adjoint_iter(const WaveArgs& a, int p, const LaunchShape& ls, const IterStreams& s, bool after_side)
 {
-    enqueue_iter<STACK, false, kTraceMinBlocks, true, REFM>(a, p, ls, st, nullptr);
+    enqueue_iter<STACK, false, kTraceMinBlocks, true, REFM>(a, p, ls, s, after_side, nullptr);
 }
 
 // resident blocks per SM of the shading build for these lights
@@ -2107,7 +2166,7 @@ int adjoint_launch_shape(const WaveArgs& a, LaunchShape& ls)
     const int dr = static_cast<int>(grad_smem_bytes(a, GRAD_ALBEDO));
     const int ds = static_cast<int>(grad_smem_bytes(a, GRAD_ALBEDO | GRAD_EMISSION));
     const int dc = static_cast<int>(grad_smem_bytes(a, GRAD_EMISSION));
-    CK(cudaFuncSetAttribute(k_regen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dr));
+    CK(cudaFuncSetAttribute(k_finish<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dr));
     CK(cudaFuncSetAttribute(k_shade<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ds));
     CK(cudaFuncSetAttribute(k_shade<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ds));
     CK(cudaFuncSetAttribute(k_shade<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ds));
@@ -2116,7 +2175,7 @@ int adjoint_launch_shape(const WaveArgs& a, LaunchShape& ls)
     const int sms = num_sms();
     int       occ_e = 0, occ_a = 0, occ_c = 0, occ_r = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_e, k_extend<STACK, false, B, REFM>, kTraceBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_regen<true>, 128, dr);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_finish<true>, 128, dr);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, k_shadow<STACK, false, B, REFM>, kTraceBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k_connect<STACK, false, B, true, REFM>, kTraceBlock, dc);
     ls.grid_trace = sms * std::max(occ_e, 1);
@@ -2197,17 +2256,17 @@ int adjoint_stream(Workspace& w, const std::vector<JobGPU>& jobs, int64_t total,
                  : (fast_only ? adjoint_launch_shape<kStack, false>(a, ls)
                               : adjoint_launch_shape<kStack, true>(a, ls));
     if (rc) return rc;
-    run.iter_launches = 4 + (ls.lights & 1) + (ls.lights >> 1);
-    auto iter = [&](cudaStream_t s2, int p, StageTimer*) {
+    run.iter_launches = 3 + (ls.lights & 1) + (ls.lights >> 1);
+    auto iter = [&](const IterStreams& s, int p, bool after_side, StageTimer*) {
         if (stack32)
-            fast_only ? enqueue_adjoint_iter<kSmallStack, false>(a, p, ls, s2)
-                      : enqueue_adjoint_iter<kSmallStack, true>(a, p, ls, s2);
+            fast_only ? enqueue_adjoint_iter<kSmallStack, false>(a, p, ls, s, after_side)
+                      : enqueue_adjoint_iter<kSmallStack, true>(a, p, ls, s, after_side);
         else
-            fast_only ? enqueue_adjoint_iter<kStack, false>(a, p, ls, s2)
-                      : enqueue_adjoint_iter<kStack, true>(a, p, ls, s2);
+            fast_only ? enqueue_adjoint_iter<kStack, false>(a, p, ls, s, after_side)
+                      : enqueue_adjoint_iter<kStack, true>(a, p, ls, s, after_side);
     };
     StageTimer timer;
-    return stream_loop(w, a, total, max_depth, false, true, st, timer, run, iter);
+    return stream_loop(w, a, ls, total, max_depth, false, false, st, timer, run, iter);
 }
 
 int render_jobs(int num_jobs, mcrt_scene* const* scenes, const mcrt_camera* cams, const mcrt_render_params* params,
@@ -2301,7 +2360,7 @@ int render_jobs(int num_jobs, mcrt_scene* const* scenes, const mcrt_camera* cams
     w.args.batch_fetch = (vb & MCRT_VARIANT_GRIDSTRIDE) ? 0 : 1;
     StageTimer  timer;
     RunResult   run;
-    run.iter_launches = 4 + (lsv.lights & 1) + (lsv.lights >> 1);
+    run.iter_launches = 3 + (lsv.lights & 1) + (lsv.lights >> 1);
     int         rc = p0.schedule == MCRT_SCHEDULE_WAVES
                          ? run_waves(w, jobs, pix_spp, total, max_depth, p0.path_chunk, stack32, regcap, count, stages,
                                      graph, lsv, st, timer, run)
@@ -2414,7 +2473,7 @@ int64_t stream_ring_entries(int64_t capacity, int max_depth, int64_t max_spp, in
     return std::min(total, (max_depth + 2) * capacity + max_spp);
 }
 
-int wave_iterations(int max_depth) { return (max_depth + 2 + 1) & ~1; }
+int wave_iterations(int max_depth) { return (max_depth + 1 + 1) & ~1; }
 
 void enqueue_render_begin(const WaveArgs& a, bool waves, int64_t limit, cudaStream_t st)
 {
@@ -2449,7 +2508,7 @@ LaunchShape launch_shape_variant(bool stack32, bool regcap, bool fast_only, int 
                : traversal_occupancy<kStack, 1, false>(occ_t, occ_a, occ_c);
     ls.fast_only = fast_only;
     ls.lights = lights;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_regen<false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_r, k_finish<false>, 128, 0);
     ls.grid_trace = sms * std::max(occ_t, 1);
     ls.grid_any = sms * std::max(occ_a, 1);
     ls.grid_connect = sms * std::max(occ_c, 1);

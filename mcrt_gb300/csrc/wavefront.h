@@ -5,19 +5,21 @@
 // Path state travels with its ray through the queues (no per-path slots): every stage
 // reads and writes its items by queue position, so all per-path traffic is coalesced.
 // One iteration (parity p = iteration & 1):
-//   k_iter_begin  zero the counters this iteration appends to; admit new paths: the
-//                 queue is topped up to its capacity from the path counter, bounded by
-//                 the admission limit (the whole render when streaming, the current wave
-//                 for the wave schedule)
-//   k_regen       finish the paths that ended in the previous iteration (their
-//                 next-event results are in): radiance into the ring, pixel resolved in
-//                 sample order when its last path finished; start the admitted paths
+//   k_admit, k_start    admit new paths and start their camera rays: the queue is topped up to
+//                 its capacity from the path counter, bounded by the admission limit.  Only
+//                 while paths wait to be admitted: a render whose paths fit one queue, and a
+//                 wave, admit all of them before their first iteration
 //   k_extend      closest hit of every ray of queue p
 //   k_shade       one vertex per ray: continuing paths to queue p ^ 1, ended paths to
 //                 the finished list p ^ 1, next-event rays to the next-event queues
 //   k_shadow, k_connect   trace the next-event rays (environment, area lights); each result
 //                 goes to the slot its path will read next (queue p ^ 1 position or
 //                 finished-list position)
+//   k_finish      finish the paths that ended: radiance into the ring, pixel resolved in
+//                 sample order when its last path finished
+// The last two need only what k_shade wrote, and nothing before the next iteration's k_shade
+// needs them: mcrt_render runs them on a second stream beside the next iteration's k_extend
+// (IterStreams).  Counters are kept per parity and cleared by the next kernel that may.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -51,20 +53,22 @@ constexpr int64_t kMaxQueue = int64_t(1) << 27;     // rays per queue (result in
 constexpr int64_t kDefaultQueue = int64_t(1) << 26;
 constexpr int64_t kMinDefaultQueue = int64_t(1) << 20;
 
-// counters of one render
+// counters of one render.  Cleared by: k_extend of parity p qcount[p ^ 1] and dcount[p ^ 1],
+// k_shade of parity p scount[p ^ 1] and fetch[p ^ 1] (each after their last reader, before their
+// next writer, also with k_shadow / k_connect / k_finish beside the next k_extend)
 struct Ctrl
 {
-    int                qcount[2];  // ray queues (by parity)
-    int                dcount[2];  // lists of finished paths (by parity)
-    int                scount[2];  // next-event queues of the current iteration: any-hit, closest-hit
-    int                new_base;   // this iteration's admitted paths: first queue position
-    int                new_count;  //   and how many
-    int                chunk;      // wave schedule: index of the current wave
-    int                fetch[3];   // rays taken so far by this iteration's k_extend, k_shadow, k_connect
-    unsigned long long next;      // index of the next path to admit
-    unsigned long long limit;     // admission limit (exclusive)
-    unsigned long long new_g;     // index of the first path admitted this iteration
-    unsigned long long finished;  // paths whose radiance reached the ring
+    int                qcount[2];     // ray queues (by parity)
+    int                dcount[2];     // lists of finished paths (by parity)
+    int                scount[2][2];  // by parity: next-event queues, any-hit and closest-hit
+    int                fetch[2][3];   // by parity: rays taken by k_extend, k_shadow, k_connect
+    int                new_base;      // admitted paths to start: first queue position
+    int                new_count;     //   and how many
+    int                chunk;         // wave schedule: index of the current wave
+    unsigned long long next;          // index of the next path to admit
+    unsigned long long limit;         // admission limit (exclusive)
+    unsigned long long new_g;         // index of the first path to start
+    unsigned long long finished;      // paths whose radiance reached the ring
 };
 
 // device pointers of one render's state (SoA, `capacity` rays per queue)
@@ -127,7 +131,7 @@ constexpr int kAdjLog = 16;
 
 struct LaunchShape
 {
-    int grid_trace, grid_any, grid_connect, grid_shade, grid_regen, grid_small, block;  // grid_any: k_shadow
+    int grid_trace, grid_any, grid_connect, grid_shade, grid_regen, grid_small, block;  // grid_any: k_shadow; grid_regen: k_start, k_finish
     bool fast_only = false;  // every job traverses in FAST mode: kernels built without the REF traversal
     int  lights = 3;         // light kinds of the jobs (1 environment, 2 area, 3 both): the k_shade build
 };

@@ -56,3 +56,26 @@ def test_streamed_hits_match_the_reference_tree(cuda_device):
     bad, _ = classify(fx["verts"], fx["rays_bounce"], fx["t_bounce"], fx["prim_bounce"], out[:, 0],
                       out[:, 3].view(np.int32))
     assert not bad.any()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("depth", [0, 1, 2, 7])
+@pytest.mark.parametrize("chunk", [0, 33 * 29 * 3, 33 * 29 * 3 - 1, 64])
+def test_admission_and_overlap_change_no_pixel(chunk, depth, graph, cuda_device):
+    """The frame whose paths are all admitted at once (as many slots as paths, and the default),
+    one slot short of that, and with 64 slots, against the wave schedule, which runs every
+    kernel after the other: the same bits, for odd and even numbers of iterations.  Both lights."""
+    import dataclasses
+    from mcrt_gb300 import GpuScene, scenes
+    desc = scenes.cfg0_scene(sphere_level=2)
+    cam = scenes.cfg0_camera(33, 29)
+    both = dataclasses.replace(desc, envmap=scenes.sky_envmap(64, 32))
+    for d in (desc, both):
+        sc = GpuScene(d)
+        kw = dict(spp=3, max_depth=depth, seed=21)
+        want, sw = sc.render(cam, schedule=1, **kw)
+        got, sg = sc.render(cam, schedule=0, path_chunk=chunk, use_graph=graph, **kw)
+        assert np.array_equal(got.view(np.int32), want.view(np.int32))
+        assert sg["rays"] == sw["rays"] and sg["paths"] == 33 * 29 * 3
+        if chunk == 0 and not graph:
+            assert sg["waves"] == depth + 1
