@@ -196,14 +196,14 @@ __device__ __forceinline__ float4 add_pending(const float4* slots, int mask, flo
 // tops queue p up with new paths (continuing rays are already in it)
 __device__ __forceinline__ void admit(Ctrl* c, int64_t capacity, int p)
 {
-    const int                q = c->qcount[p];
+    const int                q = queue_count(c->lists[p]);
     const unsigned long long avail = c->limit > c->next ? c->limit - c->next : 0ull;
     const long long          room = capacity - static_cast<long long>(q);
     const int n = room > 0 ? static_cast<int>(avail < static_cast<unsigned long long>(room) ? avail : room) : 0;
     c->new_base = q;
     c->new_count = n;
     c->new_g = c->next;
-    c->qcount[p] = q + n;
+    c->lists[p] += static_cast<unsigned long long>(n);
     c->next += static_cast<unsigned long long>(n);
 }
 
@@ -213,9 +213,9 @@ __global__ void k_render_begin(WaveArgs a, int waves, int64_t limit)
     Ctrl* c = a.ctrl;
     for (int p = 0; p < 2; ++p)
     {
-        c->qcount[p] = c->dcount[p] = 0;
-        c->scount[p][0] = c->scount[p][1] = 0;
-        c->fetch[p][0] = c->fetch[p][1] = c->fetch[p][2] = 0;
+        c->lists[p] = 0ull;
+        c->scount[0].n[p] = c->scount[1].n[p] = 0;
+        c->fetch[0].n[p] = c->fetch[1].n[p] = c->fetch[2].n[p] = 0;
     }
     c->chunk = -1;
     c->next = 0;
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(128) k_finish(WaveArgs a, int p)
 {
     extern __shared__ float sgrad[];
     const Grads        G = grads_begin<ADJ, GRAD_ALBEDO>(a, sgrad);
-    const int          n = min(a.ctrl->dcount[p], static_cast<int>(a.capacity));
+    const int          n = min(done_count(a.ctrl->lists[p]), static_cast<int>(a.capacity));
     const int          lane = threadIdx.x & 31;
     const int          warps_total = (gridDim.x * blockDim.x) >> 5;
     unsigned long long fin = 0;
@@ -567,7 +567,7 @@ struct ExtendRays : QueueFetch
     const WaveArgs& a;
     int             p;
     __device__ __forceinline__ ExtendRays(const WaveArgs& a_, int p_)
-        : QueueFetch(&a_.ctrl->fetch[p_][0], a_.batch_fetch != 0), a(a_), p(p_)
+        : QueueFetch(&a_.ctrl->fetch[0].n[p_], a_.batch_fetch != 0), a(a_), p(p_)
     {
     }
     __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.qo[p][i] : &a.qd[p][i]; }
@@ -594,13 +594,12 @@ struct ExtendRays : QueueFetch
 template <int STACK, bool COUNT, int MINB, bool REFM = true>
 __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
 {
-    const int  n = min(a.ctrl->qcount[p], static_cast<int>(a.capacity));
+    const int  n = min(queue_count(a.ctrl->lists[p]), static_cast<int>(a.capacity));
     TraceCount cnt = {0u, 0u};
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
         atomicAdd(&a.stats[0], static_cast<unsigned long long>(n));
-        a.ctrl->qcount[p ^ 1] = 0;  // (see Ctrl)
-        a.ctrl->dcount[p ^ 1] = 0;
+        a.ctrl->lists[p ^ 1] = 0ull;  // (see Ctrl)
     }
     if constexpr (!REFM && kStreamTraversal)
     {
@@ -613,7 +612,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
         __shared__ int stack[STACK * kTraceBlock];
         int*           st = stack + threadIdx.x;
         const float    inf = __int_as_float(0x7f800000);
-        for (QueueWalk w(&a.ctrl->fetch[p][0], n, a.batch_fetch != 0); w.valid(); w.next())
+        for (QueueWalk w(&a.ctrl->fetch[0].n[p], n, a.batch_fetch != 0); w.valid(); w.next())
         {
             const int i = w.i;
             if (i >= n) continue;
@@ -730,13 +729,13 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
     extern __shared__ float sgrad[];
     __shared__ int s_base[16], s_perm[kShadeWindow];
     const Grads G = grads_begin<ADJ, GRAD_ALBEDO | GRAD_EMISSION>(a, sgrad);
-    const int n = min(a.ctrl->qcount[p], static_cast<int>(a.capacity));
+    const int n = min(queue_count(a.ctrl->lists[p]), static_cast<int>(a.capacity));
     const int lane = threadIdx.x & 31;
     const int pn = p ^ 1;
     if (blockIdx.x == 0 && threadIdx.x < 3)  // (see Ctrl)
     {
-        a.ctrl->fetch[pn][threadIdx.x] = 0;
-        if (threadIdx.x < 2) a.ctrl->scount[pn][threadIdx.x] = 0;
+        a.ctrl->fetch[threadIdx.x].n[pn] = 0;
+        if (threadIdx.x < 2) a.ctrl->scount[threadIdx.x].n[pn] = 0;
     }
     // pos: the first entry of this round; windows start at multiples of kShadeWindow, and a
     // window's valid entries fill its first rounds (the sort puts entries past n last)
@@ -835,62 +834,53 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
             }
             rnew = make_float4(rp.x + Ladd.x, rp.y + Ladd.y, rp.z + Ladd.z, rp.w);
         }
-        // continuing paths -> queue p ^ 1, ended paths -> finished list p ^ 1 (ballot + popc,
-        // one atomic per warp each); dest: where this vertex's next-event results go
-        int      dest = -1;
-        unsigned live = __ballot_sync(0xffffffffu, cont);
-        if (live)
+        // continuing paths -> queue p ^ 1, ended paths -> finished list p ^ 1 (ballot + popc, one
+        // atomic per warp for both); dest: where this vertex's next-event results go
+        const unsigned     live = __ballot_sync(0xffffffffu, cont);
+        const unsigned     ended = __ballot_sync(0xffffffffu, valid && !cont);
+        unsigned long long place = 0;
+        int                dest = -1;
+        if (lane == 0 && (live | ended)) place = atomicAdd(&a.ctrl->lists[pn], list_counts(__popc(live), __popc(ended)));
+        place = __shfl_sync(0xffffffffu, place, 0);
+        if (cont)
         {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&a.ctrl->qcount[pn], __popc(live));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (cont)
+            int k = queue_count(place) + __popc(live & lanemask_lt());
+            if (k < a.capacity)
             {
-                int k = base + __popc(live & lanemask_lt());
-                if (k < a.capacity)
+                // the queues are written and read once per iteration: streaming stores
+                // leave the L2 to the tree (outdoor frame 84.6 -> 83.2 ms)
+                __stcs(&a.qo[pn][k], make_float4(phit.x, phit.y, phit.z, __int_as_float(job)));
+                __stcs(&a.qd[pn][k], make_float4(cdir.x, cdir.y, cdir.z, __int_as_float(pixel)));
+                __stcs(&a.qrad[pn][k], rnew);
+                __stcs(reinterpret_cast<unsigned long long*>(&a.qrng[pn][k]), static_cast<unsigned long long>(draws.after()));
+                if (ADJ && nlog > 0)
                 {
-                    // the queues are written and read once per iteration: streaming stores
-                    // leave the L2 to the tree (outdoor frame 84.6 -> 83.2 ms)
-                    __stcs(&a.qo[pn][k], make_float4(phit.x, phit.y, phit.z, __int_as_float(job)));
-                    __stcs(&a.qd[pn][k], make_float4(cdir.x, cdir.y, cdir.z, __int_as_float(pixel)));
-                    __stcs(&a.qrad[pn][k], rnew);
-                    __stcs(reinterpret_cast<unsigned long long*>(&a.qrng[pn][k]), static_cast<unsigned long long>(draws.after()));
-                    if (ADJ && nlog > 0)
-                    {
-                        a.qlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-                        a.qlog[pn][2 * static_cast<int64_t>(k) + 1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
-                    }
-                    dest = 4 * k;
+                    a.qlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                    a.qlog[pn][2 * static_cast<int64_t>(k) + 1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
                 }
-                else
-                {
-                    atomicOr(a.err, kErrQueue);
-                }
+                dest = 4 * k;
+            }
+            else
+            {
+                atomicOr(a.err, kErrQueue);
             }
         }
-        unsigned ended = __ballot_sync(0xffffffffu, valid && !cont);
-        if (ended)
+        else if (valid)
         {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&a.ctrl->dcount[pn], __popc(ended));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (valid && !cont)
+            int k = done_count(place) + __popc(ended & lanemask_lt());
+            if (k < a.capacity)
             {
-                int k = base + __popc(ended & lanemask_lt());
-                if (k < a.capacity)
+                a.drad[pn][k] = rnew;
+                if (ADJ && nlog > 0)
                 {
-                    a.drad[pn][k] = rnew;
-                    if (ADJ && nlog > 0)
-                    {
-                        a.dlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-                        a.dlog[pn][2 * static_cast<int64_t>(k) + 1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
-                    }
-                    dest = static_cast<int>(4 * a.capacity) + 4 * k;
+                    a.dlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                    a.dlog[pn][2 * static_cast<int64_t>(k) + 1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
                 }
-                else
-                {
-                    atomicOr(a.err, kErrQueue);
-                }
+                dest = static_cast<int>(4 * a.capacity) + 4 * k;
+            }
+            else
+            {
+                atomicOr(a.err, kErrQueue);
             }
         }
         // next-event rays: any-hit queue [0], closest-hit queue [1]; each is made, given a place
@@ -912,7 +902,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
             // a vertex's two rays side by side
             const unsigned b0 = __ballot_sync(0xffffffffu, h0), b1 = __ballot_sync(0xffffffffu, h1);
             int            base = 0;
-            if (lane == 0 && (b0 | b1)) base = atomicAdd(&a.ctrl->scount[p][0], __popc(b0) + __popc(b1));
+            if (lane == 0 && (b0 | b1)) base = atomicAdd(&a.ctrl->scount[0].n[p], __popc(b0) + __popc(b1));
             base = __shfl_sync(0xffffffffu, base, 0) + __popc(b0 & lanemask_lt()) + __popc(b1 & lanemask_lt());
             put_shadow(a, h0, base, phit, r0.d, dest, job);
             put_shadow(a, h1, base + (h0 ? 1 : 0), phit, r1.d, dest + 1, job);
@@ -931,7 +921,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                 const unsigned b = __ballot_sync(0xffffffffu, h);
                 if (!b) continue;
                 int base = 0;
-                if (lane == 0) base = atomicAdd(&a.ctrl->scount[p][1], __popc(b));
+                if (lane == 0) base = atomicAdd(&a.ctrl->scount[1].n[p], __popc(b));
                 base = __shfl_sync(0xffffffffu, base, 0) + __popc(b & lanemask_lt());
                 if (!h) continue;
                 pend |= 4 << which;
@@ -990,7 +980,7 @@ struct ShadowRays : QueueFetch
     const WaveArgs& a;
     int             p;
     __device__ __forceinline__ ShadowRays(const WaveArgs& a_, int p_)
-        : QueueFetch(&a_.ctrl->fetch[p_][1], a_.batch_fetch != 0), a(a_), p(p_)
+        : QueueFetch(&a_.ctrl->fetch[1].n[p_], a_.batch_fetch != 0), a(a_), p(p_)
     {
     }
     __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.so[0][i] : &a.sd[0][i]; }
@@ -1014,7 +1004,7 @@ template <int STACK, bool COUNT, int MINB, bool REFM = true>
 __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kAnyHitMinBlocks : MINB) k_shadow(WaveArgs a, int p)
 {
     TraceCount cnt = {0u, 0u};
-    const int  n = min(a.ctrl->scount[p][0], static_cast<int>(a.shadow_cap));
+    const int  n = min(a.ctrl->scount[0].n[p], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
     if constexpr (!REFM && kStreamTraversal)
     {
@@ -1026,7 +1016,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kAnyHitMinBlocks : MIN
     {
         __shared__ int stack[STACK * kTraceBlock];
         int*           st = stack + threadIdx.x;
-        for (QueueWalk w(&a.ctrl->fetch[p][1], n, a.batch_fetch != 0); w.valid(); w.next())
+        for (QueueWalk w(&a.ctrl->fetch[1].n[p], n, a.batch_fetch != 0); w.valid(); w.next())
         {
             const int k = w.i;
             if (k >= n) continue;
@@ -1049,7 +1039,7 @@ struct ConnectRays : QueueFetch
     const Grads&    G;
     int             p;
     __device__ __forceinline__ ConnectRays(const WaveArgs& a_, const Grads& G_, int p_)
-        : QueueFetch(&a_.ctrl->fetch[p_][2], a_.batch_fetch != 0), a(a_), G(G_), p(p_)
+        : QueueFetch(&a_.ctrl->fetch[2].n[p_], a_.batch_fetch != 0), a(a_), G(G_), p(p_)
     {
     }
     __device__ __forceinline__ const float4* src(int i, int k) const { return k == 0 ? &a.so[1][i] : &a.sd[1][i]; }
@@ -1081,7 +1071,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kConnectMinBlocks : MI
     extern __shared__ float sgrad[];
     const Grads             G = grads_begin<ADJ, GRAD_EMISSION>(a, sgrad);
     TraceCount              cnt = {0u, 0u};
-    const int               n = min(a.ctrl->scount[p][1], static_cast<int>(a.shadow_cap));
+    const int               n = min(a.ctrl->scount[1].n[p], static_cast<int>(a.shadow_cap));
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&a.stats[1], static_cast<unsigned long long>(n));
     if constexpr (!REFM && kStreamTraversal)
     {
@@ -1093,7 +1083,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kConnectMinBlocks : MI
     {
         __shared__ int stack[STACK * kTraceBlock];
         int*           st = stack + threadIdx.x;
-        for (QueueWalk w(&a.ctrl->fetch[p][2], n, a.batch_fetch != 0); w.valid(); w.next())
+        for (QueueWalk w(&a.ctrl->fetch[2].n[p], n, a.batch_fetch != 0); w.valid(); w.next())
         {
             const int k = w.i;
             if (k >= n) continue;
