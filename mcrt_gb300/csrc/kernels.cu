@@ -178,11 +178,13 @@ __device__ __forceinline__ int warp_append(int* counter, int k)
     return base + incl - k;
 }
 
-// adds a path's pending next-event results (slots[0..3], bits of `mask`) in slot order:
+// adds a path's pending next-event results (bits of `mask` over `slots`) in slot order:
 // the order in which rayTrace adds them (deterministic sum)
+template <int SLOTS = 4>
 __device__ __forceinline__ float4 add_pending(const float4* slots, int mask, float4 r)
 {
-    for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s)
         if (mask & (1 << s))
         {
             float4 v = slots[s];
@@ -382,7 +384,7 @@ __device__ __forceinline__ void finish_paths(const WaveArgs& a, const Grads& G, 
     {
         if (!valid) return;
         const int4    m = a.dmeta[p][i];
-        const float4 r = add_pending(a.nev[p] + 4 * a.capacity + 4 * static_cast<int64_t>(i), m.z, a.drad[p][i]);
+        const float4 r = add_pending(a.nev[p] + ((a.capacity + i) << a.nev_log2), m.z, a.drad[p][i]);
         ++fin;
         if (isnan3(xyz(r)) || m.w == 0) return;
         const JobGPU&    J = a.jobs[m.y];
@@ -407,7 +409,7 @@ __device__ __forceinline__ void finish_paths(const WaveArgs& a, const Grads& G, 
     if (valid)
     {
         const int4    m = a.dmeta[p][i];
-        const float4 r = add_pending(a.nev[p] + 4 * a.capacity + 4 * static_cast<int64_t>(i), m.z, a.drad[p][i]);
+        const float4 r = add_pending(a.nev[p] + ((a.capacity + i) << a.nev_log2), m.z, a.drad[p][i]);
         pixel = m.x;
         job = m.y;
         const JobGPU& J = a.jobs[job];
@@ -728,6 +730,12 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
 {
     extern __shared__ float sgrad[];
     __shared__ int s_base[16], s_perm[kShadeWindow];
+    __shared__ unsigned long long s_place[4];
+    // Result slots per path: the environment's two rays, then the area lights' two.  A scene with
+    // one kind of light has two, next to the next path's: with four, half of every 64 bytes that
+    // DRAM delivers would be another kind's (4k outdoor frame: shading 15.2 -> 14.5 ms, whole
+    // frame 76.3 -> 75.4)
+    constexpr int kSlots = LIGHTS == 3 ? 4 : 2, kAreaSlot = LIGHTS == 3 ? 2 : 0;
     const Grads G = grads_begin<ADJ, GRAD_ALBEDO | GRAD_EMISSION>(a, sgrad);
     const int n = min(queue_count(a.ctrl->lists[p]), static_cast<int>(a.capacity));
     const int lane = threadIdx.x & 31;
@@ -758,9 +766,14 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
         unsigned lw[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
         if (valid)
         {
+            // all of the path's state at once, so that its misses overlap (a result slot whose
+            // ray was not traced is read too, and not used): 4k outdoor frame 77.1 -> 76.1 ms
             float4           o4 = a.qo[p][i], d4 = a.qd[p][i];
             float4           hh = a.hits[i];
-            float4           t4 = a.qthr[p][i];
+            float4           t4 = a.qthr[p][i], r4 = a.qrad[p][i], pv[kSlots];
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s) pv[s] = a.nev[p][kSlots * static_cast<int64_t>(i) + s];
+            draws.state = a.qrng[p][i];
             float3           o = xyz(o4), d = xyz(d4);
             job = __float_as_int(o4.w);
             pixel = __float_as_int(d4.w);
@@ -774,7 +787,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
             int              prim = __float_as_int(hh.w);
             float3           Ladd = mk(0.f, 0.f, 0.f);
             // results of the previous vertex's next-event rays first, then this vertex
-            float4 rp = add_pending(a.nev[p] + 4 * static_cast<int64_t>(i), (flags >> 16) & 0xf, a.qrad[p][i]);
+            float4 rp = add_pending<kSlots>(pv, (flags >> 16) & 0xf, r4);
             float3 dl = mk(0.f, 0.f, 0.f);
             if (ADJ)
             {
@@ -824,7 +837,6 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                         else
                             atomicOr(a.err, kErrQueue);
                     }
-                    draws.state = a.qrng[p][i];
                     draws.inc = (static_cast<uint64_t>(pixel) << 1u) | 1u;
                     wi = -d;
                     nee_here = does_nee(m.type);
@@ -834,14 +846,27 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
             }
             rnew = make_float4(rp.x + Ladd.x, rp.y + Ladd.y, rp.z + Ladd.z, rp.w);
         }
-        // continuing paths -> queue p ^ 1, ended paths -> finished list p ^ 1 (ballot + popc, one
-        // atomic per warp for both); dest: where this vertex's next-event results go
-        const unsigned     live = __ballot_sync(0xffffffffu, cont);
-        const unsigned     ended = __ballot_sync(0xffffffffu, valid && !cont);
-        unsigned long long place = 0;
-        int                dest = -1;
-        if (lane == 0 && (live | ended)) place = atomicAdd(&a.ctrl->lists[pn], list_counts(__popc(live), __popc(ended)));
-        place = __shfl_sync(0xffffffffu, place, 0);
+        // continuing paths -> queue p ^ 1, ended paths -> finished list p ^ 1: one atomic per
+        // block for both (one per warp: Cornell box with a mirror 23.0 ms, per block 22.7, and
+        // the 128 neighbours stay together: start and finish of the 4k outdoor frame 4.6 -> 4.4);
+        // dest: where this vertex's next-event results go
+        const unsigned live = __ballot_sync(0xffffffffu, cont);
+        const unsigned ended = __ballot_sync(0xffffffffu, valid && !cont);
+        const int      warp = threadIdx.x >> 5;
+        int            dest = -1;
+        if (lane == 0) s_place[warp] = list_counts(__popc(live), __popc(ended));
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            const unsigned long long c0 = s_place[0], c1 = s_place[1], c2 = s_place[2], c3 = s_place[3];
+            const unsigned long long b = atomicAdd(&a.ctrl->lists[pn], c0 + c1 + c2 + c3);
+            s_place[0] = b;
+            s_place[1] = b + c0;
+            s_place[2] = b + c0 + c1;
+            s_place[3] = b + c0 + c1 + c2;
+        }
+        __syncthreads();
+        const unsigned long long place = s_place[warp];
         if (cont)
         {
             int k = queue_count(place) + __popc(live & lanemask_lt());
@@ -858,7 +883,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                     a.qlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
                     a.qlog[pn][2 * static_cast<int64_t>(k) + 1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
                 }
-                dest = 4 * k;
+                dest = kSlots * k;
             }
             else
             {
@@ -876,7 +901,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                     a.dlog[pn][2 * static_cast<int64_t>(k)] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
                     a.dlog[pn][2 * static_cast<int64_t>(k) + 1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
                 }
-                dest = static_cast<int>(4 * a.capacity) + 4 * k;
+                dest = kSlots * (static_cast<int>(a.capacity) + k);
             }
             else
             {
@@ -924,7 +949,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                 if (lane == 0) base = atomicAdd(&a.ctrl->scount[1].n[p], __popc(b));
                 base = __shfl_sync(0xffffffffu, base, 0) + __popc(b & lanemask_lt());
                 if (!h) continue;
-                pend |= 4 << which;
+                pend |= (1 << kAreaSlot) << which;
                 if (base >= a.shadow_cap)
                 {
                     atomicOr(a.err, kErrQueue);
@@ -934,14 +959,14 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
                 __stcs(&a.so[1][base], make_float4(phit.x, phit.y, phit.z, r.tterm));
                 __stcs(&a.sd[1][base], make_float4(r.d.x, r.d.y, r.d.z, r.tmax));
                 a.sv[base] = r.val;
-                a.sm[base] = make_int4(dest + 2 + which, r.type | (r.light << 2), pixel, job);
+                a.sm[base] = make_int4(dest + kAreaSlot + which, r.type | (r.light << 2), pixel, job);
             }
         }
         // the path's entry records which result slots will hold one
         if (dest >= 0 && cont)
-            __stcs(&a.qthr[pn][dest >> 2], make_float4(T2.x, T2.y, T2.z, __int_as_float(flags2 | (pend << 16))));
+            __stcs(&a.qthr[pn][dest / kSlots], make_float4(T2.x, T2.y, T2.z, __int_as_float(flags2 | (pend << 16))));
         else if (dest >= 0)
-            a.dmeta[pn][(dest >> 2) - a.capacity] = make_int4(pixel, job, pend, ADJ ? nlog : 0);
+            a.dmeta[pn][dest / kSlots - a.capacity] = make_int4(pixel, job, pend, ADJ ? nlog : 0);
         pos += 128;
         if (pos % kShadeWindow == 0) pos += (gridDim.x - 1) * kShadeWindow;
     }
@@ -1689,8 +1714,10 @@ struct StageTimer
 // 2 shade, 3 next-event rays (a timed iteration runs on one stream).  after_side: the
 // iteration before left work on the side stream.
 template <int STACK, bool COUNT, int MINB, bool ADJ = false, bool REFM = true>
-void enqueue_iter(const WaveArgs& a, int p, const LaunchShape& ls, const IterStreams& s, bool after_side, StageTimer* tm)
+void enqueue_iter(const WaveArgs& args, int p, const LaunchShape& ls, const IterStreams& s, bool after_side, StageTimer* tm)
 {
+    WaveArgs a = args;
+    a.nev_log2 = ls.lights == 3 ? 2 : 1;  // result slots per path (see k_shade)
     // adjoint: each kernel's shared gradient slices (0 for the forward)
     const size_t dr = ADJ ? grad_smem_bytes(a, GRAD_ALBEDO) : 0;
     const size_t ds = ADJ ? grad_smem_bytes(a, GRAD_ALBEDO | GRAD_EMISSION) : 0;

@@ -107,9 +107,10 @@ struct WaveArgs
     // finished paths by parity: radiance (w = sample), {pixel, job, pending mask, 0}
     float4* drad[2];
     int4*   dmeta[2];
-    // next-event results by parity: [4 i + s] for queue position i, [4 capacity + 4 j + s]
-    // for finished-list position j
+    // next-event results by parity, s of 2 ^ nev_log2 slots: [(i << nev_log2) + s] for queue
+    // position i, [((capacity + j) << nev_log2) + s] for finished-list position j
     float4* nev[2];
+    int     nev_log2;  // 2 with both kinds of light, else 1 (set with the shading build)
     // next-event queues; tmin is kEpsRay for all.
     // [0] any-hit: origin + result index, direction + job (int bits); the value an unoccluded
     //     ray adds is already in its result slot

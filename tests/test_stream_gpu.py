@@ -79,3 +79,25 @@ def test_admission_and_overlap_change_no_pixel(chunk, depth, graph, cuda_device)
         assert sg["rays"] == sw["rays"] and sg["paths"] == 33 * 29 * 3
         if chunk == 0 and not graph:
             assert sg["waves"] == depth + 1
+
+
+@pytest.mark.parametrize("chunk", [1, 127, 129, 511, 513, 0])
+@pytest.mark.parametrize("kind", ["environment", "area", "both"])
+def test_light_kinds_alone_and_beside_the_others(kind, chunk, cuda_device):
+    """A scene with one kind of light keeps two next-event results per path, one with both (or a
+    batch that has both) four: the same image alone as in a batch beside the other kinds, with
+    queues around a block and around a sorted window (path_chunk paths in flight).  The bound is
+    that of the other batch test: the builds may round differently."""
+    import dataclasses
+    from mcrt_gb300 import GpuScene, render_batch, scenes
+    area = scenes.cfg0_scene(sphere_level=1)
+    descs = {"area": (area, scenes.cfg0_camera(13, 11)),
+             "environment": (scenes.cfg1_scene(level=2, env_size=(64, 32)), scenes.cfg1_camera(13, 11)),
+             "both": (dataclasses.replace(area, envmap=scenes.sky_envmap(64, 32)), scenes.cfg0_camera(13, 11))}
+    p = dict(spp=1 if chunk == 1 else 4, max_depth=4, rr_depth=2, seed=17, path_chunk=chunk)
+    names = [kind] + [k for k in descs if k != kind]
+    gs = {k: GpuScene(descs[k][0]) for k in names}
+    alone, _ = gs[kind].render(descs[kind][1], **p)
+    outs, _ = render_batch([gs[k] for k in names], [descs[k][1] for k in names], [p] * 3)
+    assert alone.max() > 0
+    np.testing.assert_allclose(outs[0], alone, rtol=1e-5, atol=1e-6)
