@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
     __shared__ unsigned long long s_place[4];
     // Result slots per path: the environment's two rays, then the area lights' two.  A scene with
     // one kind of light has two, next to the next path's: with four, half of every 64 bytes that
-    // DRAM delivers would be another kind's (4k outdoor frame: shading 15.2 -> 14.5 ms, whole
+    // DRAM delivers would be another kind's (outdoor frame: shading 15.2 -> 14.5 ms, whole
     // frame 76.3 -> 75.4)
     constexpr int kSlots = LIGHTS == 3 ? 4 : 2, kAreaSlot = LIGHTS == 3 ? 2 : 0;
     const Grads G = grads_begin<ADJ, GRAD_ALBEDO | GRAD_EMISSION>(a, sgrad);
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
         if (valid)
         {
             // all of the path's state at once, so that its misses overlap (a result slot whose
-            // ray was not traced is read too, and not used): 4k outdoor frame 77.1 -> 76.1 ms
+            // ray was not traced is read too, and not used): outdoor frame 77.1 -> 76.1 ms
             float4           o4 = a.qo[p][i], d4 = a.qd[p][i];
             float4           hh = a.hits[i];
             float4           t4 = a.qthr[p][i], r4 = a.qrad[p][i], pv[kSlots];
@@ -848,7 +848,7 @@ __global__ void __launch_bounds__(128, LIGHTS == 1 ? kShadeBlocksEnv : kShadeBlo
         }
         // continuing paths -> queue p ^ 1, ended paths -> finished list p ^ 1: one atomic per
         // block for both (one per warp: Cornell box with a mirror 23.0 ms, per block 22.7, and
-        // the 128 neighbours stay together: start and finish of the 4k outdoor frame 4.6 -> 4.4);
+        // the 128 neighbours stay together: start and finish of the outdoor frame 4.6 -> 4.4);
         // dest: where this vertex's next-event results go
         const unsigned live = __ballot_sync(0xffffffffu, cont);
         const unsigned ended = __ballot_sync(0xffffffffu, valid && !cont);
@@ -1091,7 +1091,7 @@ struct ConnectRays : QueueFetch
 };
 
 template <int STACK, bool COUNT, int MINB, bool ADJ, bool REFM = true>
-__global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? kConnectMinBlocks : MINB) k_connect(WaveArgs a, int p)
+__global__ void __launch_bounds__(kTraceBlock, MINB > 1 ? (ADJ ? kConnectAdjMinBlocks : kConnectMinBlocks) : MINB) k_connect(WaveArgs a, int p)
 {
     extern __shared__ float sgrad[];
     const Grads             G = grads_begin<ADJ, GRAD_EMISSION>(a, sgrad);

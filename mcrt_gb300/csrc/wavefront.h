@@ -42,11 +42,17 @@ constexpr int kSmallStack = 32;
 // 23.3, at 9 23.5.  With the lanes refilled (trace_stream) more warps than this no longer help.
 // Next-event rays to area lights: 7 blocks (72 registers) 0.68 ms per Cornell frame, 8 0.72.
 constexpr int kTraceMinBlocks = 8;
+// The adjoint's build: 9 (56 registers).  It adds each ray's emission derivative to its block's
+// sums, lanes of one emitter one after the other, and more warps hide that: the gradients of a
+// 512x512 Cornell box with a mirror 22.2 ms forward and adjoint, at 7 22.6.  More blocks also
+// mean shorter float sums, and the sum's rounding shows in the gradient: between 7 and 9 blocks
+// dL/dE differs by 2e-5 to 4e-5 relative, between runs of one build by 5e-6.
 constexpr int kConnectMinBlocks = 7;
+constexpr int kConnectAdjMinBlocks = 9;
 constexpr int kAnyHitMinBlocks = 10;
 constexpr int kMaxDepth = 62;
 constexpr int64_t kMaxQueue = int64_t(1) << 27;     // rays per queue (result indices stay in int)
-// Streaming schedule default: 64 M rays (49 GB of queues).  Per cfg1 frame (67 M paths):
+// Streaming schedule default: 64 M rays (45 GB of queues).  Per cfg1 frame (67 M paths):
 // 1 / 2 / 4 / 8 / 16 / 32 / 64 M rays 184.6 / 146.9 / 128.1 / 118.3 / 113.4 / 111.4 /
 // 109.5 ms -- fewer, longer launches amortise each launch's ramp and tail.  If its
 // allocation fails the default halves itself, down to kMinDefaultQueue.
