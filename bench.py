@@ -111,11 +111,11 @@ class ClockSampler:
 
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per extension ray of
 # k_extend on the large configuration, from a capture of three full-queue launches of a
-# reduced case (2,097,152-ray queue, same scene and frame: 337.9 MB per launch); the bench
+# reduced case (2,097,152-ray queue, same scene and frame: 277.4 MB per launch); the bench
 # scales it by the extension rays of an average launch of the measured configuration.  An
 # upper bound for larger launches, whose rays share more of the tree lines fetched.  Keyed
 # by the node size of the traversal (64: two-child nodes).
-K_EXTEND_DRAM_BYTES_PER_RAY = {64: 161.1}
+K_EXTEND_DRAM_BYTES_PER_RAY = {64: 132.3}
 
 
 # rows of the cfg0 / cfg1 frames the CPU port renders for cpu_baseline and --impl reference
@@ -577,8 +577,10 @@ def main():
     # algorithmic bytes of the two traversal kernels: a counting render of the same seeds.
     # k_extend per extension ray: one node fetch per node visited (96 B for the eight-child
     # nodes of the FAST traversal, the sectors a visit touches), 48 B per triangle tested,
-    # 32 B ray + 16 B hit; k_connect per next-event ray: nodes/triangles as above, 64 B ray +
-    # payload + meta in, 16 B result out.  Both kernels launch once per iteration.
+    # 32 B ray + 16 B hit; the next-event kernels per ray: nodes/triangles as above; environment
+    # rays (k_shadow) 32 B in and the 16-B slot an occluded ray clears, area-light rays
+    # (k_connect) 64 B ray + payload + meta in, 16 B result out.  Each launches once per iteration.
+    nee_io = 32 + 16 if args.workload in ("cfg1", "cfg4") else 64 + 16
     _, sc_cnt = sc.render(cam, seed=0, out=out, profile=PROFILE_COUNT, **kw)
     nb = sc_cnt["node_bytes"]
     # the same counts by bounce class: a depth-0 counting render of the same seeds traces
@@ -596,17 +598,17 @@ def main():
                              sc_cnt["extension_rays"] - sc_prim["extension_rays"]),
         "next_event": {**per_ray(sc_cnt["nee_nodes"], sc_cnt["nee_tris"], sc_cnt["shadow_rays"]),
                        "bytes_per_ray": round((nb * sc_cnt["nee_nodes"] + 48 * sc_cnt["nee_tris"])
-                                              / max(sc_cnt["shadow_rays"], 1) + 80, 1)},
+                                              / max(sc_cnt["shadow_rays"], 1) + nee_io, 1)},
         "note": "counting build (MCRT_PROFILE_COUNT), same seeds as the timed steps; bytes per ray as the "
                 "roofline's algorithmic bytes (ray in + hit or result out included)",
     }
     ext_bytes = nb * sc_cnt["ext_nodes"] + 48 * sc_cnt["ext_tris"] + (32 + 16) * sc_cnt["extension_rays"]
-    nee_bytes = nb * sc_cnt["nee_nodes"] + 48 * sc_cnt["nee_tris"] + (64 + 16) * sc_cnt["shadow_rays"]
+    nee_bytes = nb * sc_cnt["nee_nodes"] + 48 * sc_cnt["nee_tris"] + nee_io * sc_cnt["shadow_rays"]
     launches_per_render = max(extend_launches, 1)
     kernels = {
         "k_extend (closest-hit traversal of extension rays)": (ext_bytes, stage_ms[1], sc_cnt["extension_rays"],
                                                                 sc_cnt["ext_nodes"], sc_cnt["ext_tris"]),
-        "k_connect (next-event rays: any-hit / bounded closest-hit)": (nee_bytes, stage_ms[3], sc_cnt["shadow_rays"],
+        "k_shadow / k_connect (next-event rays: any-hit / bounded closest-hit)": (nee_bytes, stage_ms[3], sc_cnt["shadow_rays"],
                                                                         sc_cnt["nee_nodes"], sc_cnt["nee_tris"]),
     }
     dom = max(kernels, key=lambda k: kernels[k][1])
@@ -685,10 +687,10 @@ def main():
                                         "per launch, best of 3 (the traversal's node and triangle reads are served "
                                         "by L2; ncu shows DRAM a few % busy)",
                          "limiter": "dependent-load latency and SIMT divergence (ncu: long-scoreboard stalls, "
-                                    "about 10 of 32 lanes active per instruction)",
+                                    "about 16 of 32 lanes active per instruction)",
                          "traffic": None if traffic is None else int(traffic),
                          "traffic_unit": "DRAM bytes per launch: ncu read + write per extension ray of a "
-                                         "2 M-ray-queue case (161.1 B) times this configuration's rays per launch "
+                                         "2 M-ray-queue case (132.3 B) times this configuration's rays per launch "
                                          "(an upper bound: larger launches share more tree lines)",
                          "algorithmic_bytes_per_launch": int(per_launch_bytes),
                          "avg_launch_ms": round(avg_launch_ms, 4),

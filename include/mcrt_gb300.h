@@ -178,7 +178,9 @@ typedef struct mcrt_render_params {
 /* variant 0 = default policy (STACK32 when the BVH is shallow enough, REGCAP);
  * MCRT_VARIANT_EXPLICIT | bits = exactly the given bits (for tuning) */
 #define MCRT_VARIANT_STACK32 1  /* 32-entry shared-memory stacks (16 KB/block) when the BVH is shallow enough */
-#define MCRT_VARIANT_REGCAP 2   /* cap registers at 56 so 9 blocks of 128 threads fit an SM */
+#define MCRT_VARIANT_REGCAP 2   /* cap the traversal kernels' registers (64, 48 and 72 for
+                                   extension, any-hit and area-light rays: 8, 10 and 7 blocks of
+                                   128 threads per SM) */
 #define MCRT_VARIANT_EXPLICIT 4 /* use the bits as given instead of the default policy */
 #define MCRT_VARIANT_GRIDSTRIDE 8 /* traversal kernels: static grid stride instead of warps taking
                                      32-ray batches from a counter */
@@ -191,10 +193,12 @@ typedef struct mcrt_render_stats {
     int64_t paths;
     int64_t extension_rays;
     int64_t shadow_rays;
-    int32_t waves;       /* WAVES: waves; STREAM: iterations (regen + extend + shade + connect) */
+    int32_t waves;       /* WAVES: waves; STREAM: iterations (start + extend + shade + next-event
+                            rays + finish) */
     int32_t kernel_launches;
     float   device_ms;   /* CUDA-event time of the kernels (excludes host copies) */
-    float   stage_ms[4]; /* MCRT_PROFILE_STAGES: begin+raygen+resolve, extend, shade, connect */
+    float   stage_ms[4]; /* MCRT_PROFILE_STAGES: admit+start+finish, extend, shade, next-event
+                            rays (the stages one after the other, without overlap) */
     int32_t extend_launches;
     int64_t ext_nodes;   /* MCRT_PROFILE_COUNT: nodes fetched / triangles tested by extension */
     int64_t ext_tris;    /* rays, and by next-event rays */
@@ -352,7 +356,7 @@ int mcrt_autotune(int32_t num_jobs, mcrt_scene* const* scenes, const mcrt_camera
  * that reserve their memory at start-up under a hard budget.  Same image as mcrt_render
  * with ptr_mode = MCRT_PTR_DEVICE; rgb_out must be device memory.  It always runs the
  * WAVES schedule (params->schedule and params->path_chunk are not used).
- * Scratch: one fixed file-scope device array of about 50 MB, held by every GPU that loads
+ * Scratch: one fixed file-scope device array of about 46 MB, held by every GPU that loads
  * the library's module until the process exits; at most 65,536 path slots per wave
  * (spp <= 65,536) and 65,536 waves per call, larger requests fail with
  * MCRT_ERR_INVALID_ARGUMENT.  The first call on a device looks up the array's device

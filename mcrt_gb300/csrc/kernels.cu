@@ -640,8 +640,8 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
 // are made: each ray is written to its queue as it is made (an array of up to four lay in local
 // memory before, with the vertex's 14 random numbers), and a number is drawn where it is used
 // (VertexDraws).  Outdoor frame 18.7 -> 16.1 ms of shading (67 M paths; sincosf for the sine and
-// cosine of one angle is 0.7 of that), a 512x512 Cornell frame with 256 albedos forward and
-// adjoint 24.7 -> 23.5 ms.
+// cosine of one angle is 0.7 of that; with two result slots per path and the state loaded at
+// once 14.5 now), a 512x512 Cornell frame with 256 albedos forward and adjoint 24.7 -> 23.5 ms.
 // Registers: environment-only build at 7 / 8 / 9 / 10 blocks per SM 17.6 / 16.8 / 17.0 / 17.9 ms
 // (before sincosf; 8 views forward + adjoint 28.9 / 28.8 / 29.0 / 29.4), builds with area
 // lights at 6 / 7 / 8 / 9 0.65 / 0.64 / 0.67 / 0.70 ms per Cornell frame.

@@ -10,7 +10,7 @@
 //
 // The wavefront needs scratch memory for its queues, its per-path ring and its counters.
 // Here it lives in a file-scope static __device__ array of fixed size
-// (kNoAllocScratchBytes, about 50 MB): no cudaMalloc, cudaFree, event, graph or library
+// (kNoAllocScratchBytes, about 46 MB): no cudaMalloc, cudaFree, event, graph or library
 // allocation happens in the call.  The array belongs to this file's module, so every GPU
 // that loads it holds it until the process exits.  The render runs the wave schedule with
 // waves of at most kNoAllocPaths paths and at most kNoAllocWaves waves; requests beyond
