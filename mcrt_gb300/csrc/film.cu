@@ -160,9 +160,12 @@ __host__ __device__ __forceinline__ unsigned float_from(int m, int e)
                         : static_cast<unsigned>(m);  // subnormal (e is 1)
 }
 
-// what adding x (bits, finite and >= 0) does to m in binade e
+// what adding x (bits, finite and >= 0) does to m in binade e.  -0.0 is among them and adds nothing;
+// its sign bit read as part of the exponent would put it far above every sum, and chunk_add would
+// spend a pass of the block on each (a 64x64 image of them 8.0 ms instead of 0.13).
 __host__ __device__ __forceinline__ Inc inc_of(unsigned bits, int e)
 {
+    bits &= 0x7fffffffu;
     const int shift = e - binade(bits), mant = multiple(bits);
     Inc       r;
     if (shift < 0)
