@@ -2103,7 +2103,13 @@ int stream_loop(Workspace& w, const WaveArgs& a, const LaunchShape& ls, int64_t 
             return fail(MCRT_ERR_INTERNAL, "streaming render did not finish within its iteration bound");
         }
     }
-    if (e == cudaSuccess && !graph && s.side != st) e = cudaStreamWaitEvent(st, w.join, 0);
+    // `st` goes on after all of the side stream's work, the copy of the last poll among it (the
+    // iteration's own join lies before that copy, which a following render's polls could meet)
+    if (e == cudaSuccess && !graph && s.side != st)
+    {
+        e = cudaEventRecord(w.join, s.side);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, w.join, 0);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(run.e1, st);
     if (e == cudaSuccess && graph) e = cudaStreamSynchronize(st);  // before the graph is destroyed
     if (poll_ev[0]) cudaEventDestroy(poll_ev[0]);
