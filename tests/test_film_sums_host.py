@@ -1,5 +1,6 @@
 """The arithmetic of the parallel ordered float sums, on the CPU (film.cu's increments are host and
-device code): -0.0 adds nothing, and the sum composed from increments has the bits of the plain loop."""
+device code): the sum composed from increments has the bits of the plain loop, on sequences whose
+ties are counted, at even and at odd multiples of the sum's unit; and -0.0 adds nothing."""
 import ctypes
 import os
 import subprocess
@@ -57,3 +58,22 @@ def test_signed_zeros_take_no_run_out_of_the_scheme(run, sums):
     got, redone, _ = _ordered(sums, x, run)
     assert got.view(np.int32) == want.view(np.int32) == _loop(x).view(np.int32)
     assert redone == plain
+
+
+@pytest.mark.parametrize("run", [1, 7, 8, 256, 1000])
+@pytest.mark.parametrize("first,low", [(2.0 ** 20, 10), (2.0 ** 23, 12), (2.0 ** -3, 8), (3.0 * 2.0 ** 40, 9)])
+def test_ties_go_to_even_from_either_parity(first, low, run, sums):
+    """Odd multiples of half an ulp of the first addend, mixed with whole ulps and with values
+    beside the tie: the sum stays in the first addend's binade, so each odd one is a tie."""
+    rng = np.random.default_rng(low)
+    half = np.spacing(np.float32(first)).astype(np.float64) / 2
+    k = rng.integers(0, 2 ** low, 6000)
+    x = (k * half).astype(np.float32)
+    beside = rng.uniform(size=x.size) < 0.2
+    x[beside] = np.nextafter(x[beside], np.float32(np.inf))
+    x = np.concatenate([[np.float32(first)], x]).astype(np.float32)
+    assert x.astype(np.float64).sum() < 2.0 ** (np.floor(np.log2(first)) + 1)
+    got, redone, ties = _ordered(sums, x, run)
+    assert got.view(np.int32) == _loop(x).view(np.int32)
+    assert redone == 1  # the first run only, which holds the first addend
+    assert min(ties) > 500, ties
