@@ -2055,10 +2055,13 @@ int stream_loop(Workspace& w, const WaveArgs& a, const LaunchShape& ls, int64_t 
         one(c, 0, false, false, nullptr);
         one(c, 1, false, true, nullptr);
         cudaError_t e = cudaStreamWaitEvent(cap, w.join, 0);
-        if (e == cudaSuccess) e = cudaStreamEndCapture(cap, &g);
+        // ended in any case: the workspace's side stream has joined the capture and would stay in it
+        const cudaError_t ended = cudaStreamEndCapture(cap, &g);
+        if (e == cudaSuccess) e = ended;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
         if (e != cudaSuccess)
         {
+            cudaGetLastError();  // reported here, not by the next render's launches
             release_graph();
             return fail(MCRT_ERR_CUDA, std::string("stream graph: ") + cudaGetErrorString(e));
         }

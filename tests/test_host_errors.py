@@ -1,0 +1,46 @@
+"""Host code after a CUDA call failed: the error is returned, nothing half made is kept, and the next
+call works.  On the CPU, over a stand-in for the CUDA runtime whose calls fail on request
+(fake_cuda)."""
+import pytest
+
+import fake_cuda
+
+
+@pytest.fixture(scope="module")
+def built(tmp_path_factory):
+    return fake_cuda.build(str(tmp_path_factory.mktemp("fake")))
+
+
+@pytest.fixture
+def cuda(built, monkeypatch):
+    return fake_cuda.Fake(built, monkeypatch)
+
+
+def _scene():
+    from mcrt_gb300 import GpuScene, scenes
+    return GpuScene(scenes.cfg0_scene(sphere_level=1)), scenes.cfg0_camera(16, 12)
+
+
+KW = dict(spp=2, max_depth=3)
+PATHS = 16 * 12 * 2
+INVALID_VALUE = 1
+
+
+@pytest.mark.parametrize("function", ["cudaStreamWaitEvent", "cudaLaunchKernel", "cudaEventRecord"])
+@pytest.mark.parametrize("nth", [1, 2, 3, 4])
+def test_a_capture_that_fails_is_ended(function, nth, cuda):
+    """A call that fails while the iterations are captured fails the render; the capture, which the
+    workspace's side stream has joined, is ended, and the next render runs."""
+    from mcrt_gb300 import McrtError
+    scene, cam = _scene()
+    cuda.polls_read(PATHS)
+    # calls before the capture: two kernels, one event
+    before = {"cudaLaunchKernel": 2, "cudaEventRecord": 1}.get(function, 0)
+    cuda.fail(function, before + nth, INVALID_VALUE)
+    with pytest.raises(McrtError):
+        scene.render(cam, use_graph=True, path_chunk=64, **KW)
+    assert cuda.lib.fake_fails_left() == 0
+    assert cuda.lib.fake_open_captures() == 0
+    for graph in (False, True):
+        scene.render(cam, use_graph=graph, path_chunk=64, **KW)
+        assert cuda.lib.fake_pending() == 0
