@@ -2310,6 +2310,7 @@ int render_jobs(int num_jobs, mcrt_scene* const* scenes, const mcrt_camera* cams
     DeviceWorkspace&            dw = device_workspace(owner->device);
     std::lock_guard<std::mutex> wlock(dw.mu);
     CK(cudaSetDevice(owner->device));
+    (void)cudaGetLastError();  // an earlier call's error is not this render's: its launches are checked below
     const mcrt_render_params& p0 = params[0];
     int                       ptr_mode = p0.ptr_mode;
     int                       bvh_depth = 0;
@@ -3033,6 +3034,7 @@ static int adjoint_jobs(int num_jobs, mcrt_scene* const* scenes, const mcrt_came
     DeviceWorkspace&            dw = device_workspace(owner->device);
     std::lock_guard<std::mutex> wlock(dw.mu);
     CK(cudaSetDevice(owner->device));
+    (void)cudaGetLastError();  // an earlier call's error is not this render's: its launches are checked below
     std::vector<void*> temp;
     auto               cleanup = [&]() {
         for (void* t : temp) cudaFree(t);

@@ -1,9 +1,11 @@
 """Host code after a CUDA call failed: the error is returned, nothing half made is kept, and the next
 call works.  On the CPU, over a stand-in for the CUDA runtime whose calls fail on request
 (fake_cuda)."""
+import numpy as np
 import pytest
 
 import fake_cuda
+from mcrt_gb300 import McrtError
 
 
 @pytest.fixture(scope="module")
@@ -23,7 +25,7 @@ def _scene():
 
 KW = dict(spp=2, max_depth=3)
 PATHS = 16 * 12 * 2
-INVALID_VALUE = 1
+INVALID_VALUE, OUT_OF_MEMORY = 1, 2
 
 
 @pytest.mark.parametrize("function", ["cudaStreamWaitEvent", "cudaLaunchKernel", "cudaEventRecord"])
@@ -31,7 +33,6 @@ INVALID_VALUE = 1
 def test_a_capture_that_fails_is_ended(function, nth, cuda):
     """A call that fails while the iterations are captured fails the render; the capture, which the
     workspace's side stream has joined, is ended, and the next render runs."""
-    from mcrt_gb300 import McrtError
     scene, cam = _scene()
     cuda.polls_read(PATHS)
     # calls before the capture: two kernels, one event
@@ -44,3 +45,22 @@ def test_a_capture_that_fails_is_ended(function, nth, cuda):
     for graph in (False, True):
         scene.render(cam, use_graph=graph, path_chunk=64, **KW)
         assert cuda.lib.fake_pending() == 0
+
+
+def _render(scene, cam, adjoint):
+    if adjoint:
+        scene.render_adjoint(cam, 2, 3, np.zeros((12, 16, 3), np.float32), 1, 1, path_chunk=64)
+    else:
+        scene.render(cam, path_chunk=64, **KW)
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_a_failed_render_does_not_fail_the_next(adjoint, cuda):
+    """The runtime keeps the error of a failed allocation; the next render's check of its own
+    launches must not report it."""
+    scene, cam = _scene()
+    cuda.polls_read(PATHS)
+    cuda.fail("cudaMalloc", 1, OUT_OF_MEMORY)  # the image's or the gradients' device copy
+    with pytest.raises(McrtError):
+        _render(scene, cam, adjoint)
+    _render(scene, cam, adjoint)
