@@ -1663,16 +1663,14 @@ int ensure_workspace(Workspace& w, int64_t capacity, int64_t ring, int num_jobs,
         CK(cudaMalloc(&w.chunk_table, sizeof(int64_t) * (num_chunks + 1)));
         w.chunks_cap = num_chunks + 1;
     }
-    if (!w.ctrl)
-    {
-        CK(cudaMalloc(&w.ctrl, sizeof(Ctrl)));
-        CK(cudaMalloc(&w.stats, sizeof(unsigned long long) * 8));
-        CK(cudaMalloc(&w.err, sizeof(int)));
-        CK(cudaMallocHost(&w.h_poll, 2 * sizeof(unsigned long long)));
-        CK(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
-    }
+    // one by one: a call that failed here has left the later ones to be made
+    if (!w.ctrl) CK(cudaMalloc(&w.ctrl, sizeof(Ctrl)));
+    if (!w.stats) CK(cudaMalloc(&w.stats, sizeof(unsigned long long) * 8));
+    if (!w.err) CK(cudaMalloc(&w.err, sizeof(int)));
+    if (!w.h_poll) CK(cudaMallocHost(&w.h_poll, 2 * sizeof(unsigned long long)));
+    if (!w.side) CK(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
+    if (!w.fork) CK(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
+    if (!w.join) CK(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
     if (w.block) carve_queues(w.args, w.block, w.capacity);
     if (w.ring_block) carve_ring(w.args, w.ring_block, w.ring);
     w.args.ctrl = w.ctrl;

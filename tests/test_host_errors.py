@@ -64,3 +64,21 @@ def test_a_failed_render_does_not_fail_the_next(adjoint, cuda):
     with pytest.raises(McrtError):
         _render(scene, cam, adjoint)
     _render(scene, cam, adjoint)
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+@pytest.mark.parametrize("function,nth", [("cudaMalloc", k) for k in range(1, 9)] + [("cudaHostAlloc", 1)] +
+                         [("cudaStreamCreateWithFlags", 1), ("cudaEventCreateWithFlags", 1),
+                          ("cudaEventCreateWithFlags", 2)])
+def test_a_working_block_that_could_not_be_made_whole_is_completed(function, nth, adjoint, cuda):
+    """Each allocation of the first render on a device fails in turn: the render reports it, and the
+    next one makes what is missing (no null pointer, stream or event reaches the runtime)."""
+    scene, cam = _scene()
+    cuda.polls_read(PATHS)
+    cuda.fail(function, nth, OUT_OF_MEMORY)
+    with pytest.raises(McrtError):
+        _render(scene, cam, adjoint)
+    assert cuda.lib.fake_fails_left() == 0
+    _render(scene, cam, adjoint)
+    assert cuda.lib.fake_nulls() == 0
+    assert cuda.lib.fake_pending() == 0
