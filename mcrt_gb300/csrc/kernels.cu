@@ -2735,6 +2735,7 @@ void* thread_scratch(int device, size_t bytes, bool& failed)
     ThreadScratch& b = buffers[device];
     if (!b.ptr && cudaMalloc(&b.ptr, kThreadScratchMax) != cudaSuccess)
     {
+        cudaGetLastError();  // the caller is told by `failed`; its own launch check must not find it
         b.ptr = nullptr;
         failed = true;
     }

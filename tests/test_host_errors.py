@@ -82,3 +82,26 @@ def test_a_working_block_that_could_not_be_made_whole_is_completed(function, nth
     _render(scene, cam, adjoint)
     assert cuda.lib.fake_nulls() == 0
     assert cuda.lib.fake_pending() == 0
+
+
+def test_tone_mapping_without_kept_scratch_uses_its_own(cuda):
+    """The host thread's kept scratch cannot be allocated: Reinhard takes a smaller buffer of its
+    own and the call succeeds (the failed allocation's error is not taken for a launch's)."""
+    from mcrt_gb300 import film
+    img = np.ones((5, 7, 3), np.float32)
+    cuda.fail("cudaMalloc", 2, OUT_OF_MEMORY)  # after the image's device copy
+    film.tonemap(img, "reinhard")
+    assert cuda.lib.fake_fails_left() == 0
+    assert len(cuda.kernels()) == 4
+    assert cuda.lib.fake_pending() == 0
+
+
+def test_a_failed_host_trace_does_not_fail_the_next(cuda):
+    scene, _ = _scene()
+    rays = np.zeros((3, 8), np.float32)
+    cuda.fail("cudaMalloc", 1, OUT_OF_MEMORY)  # the kept scratch
+    with pytest.raises(McrtError):
+        scene.trace_closest(rays)
+    assert cuda.lib.fake_fails_left() == 0
+    scene.trace_closest(rays)
+    assert cuda.lib.fake_pending() == 0
