@@ -1,7 +1,7 @@
 // CUDA kernels (sm_103a) and the C ABI of mcrt_gb300.h.
 //
 // Kernels:
-//   k_trace<ANY, MODE, STACK, MINB>  batch closest/any-hit queries (SceneBVH::intersect / occluded)
+//   k_trace<ANY, MODE, STACK, MINB, STREAM>  batch closest/any-hit queries (SceneBVH::intersect / occluded)
 //   wavefront iterations (wavefront.h; all graph-capturable: every count is read from
 //   device memory, grids are fixed):
 //     k_render_begin, k_wave_next, k_admit   counters and admission
@@ -42,9 +42,20 @@ namespace mcrt {
 // ---------------------------------------------------------------------------
 // batch trace
 // ---------------------------------------------------------------------------
-// FAST mode (MODE 0): trace_stream; STACK / MINB as the wavefront's builds, 32-entry stacks
-// when the tree is shallow enough, registers capped for MINB blocks per SM.  REF mode (MODE 1):
-// each warp takes the next 32 consecutive rays from a counter until the batch is done.
+// FAST mode (MODE 0): STACK / MINB as the wavefront's builds, 32-entry stacks when the tree is
+// shallow enough, registers capped for MINB blocks per SM.  STREAM: trace_stream, for batches with
+// more rays than the GPU holds lanes; else, and in REF mode (MODE 1), each warp takes the next 32
+// consecutive rays from a counter until the batch is done.
+//
+// Where every warp gets one batch at most (closest hits up to 155,648 rays, any hits up to 194,560),
+// no lane is ever refilled: the warp's longest ray is its time, and trace_stream's vote per node
+// step only makes that ray's chain longer.  Kernel us, one batch a warp / streamed, incoherent rays:
+// 1.3 M triangles 32 rays 23.5 / 27.7, 2,048 83.7 / 89.9, 20,011 151.8 / 162.2, 100,000 227 / 239;
+// Cornell box 32 rays 10.2 / 12.5, 2,048 21.4 / 24.4, 100,000 33.0 / 37.8.  Camera rays side by side
+// are the exception: 20,011 to 100,000 of them take 152-203 / 139-202 and 34-37 / 32-35.  Above the
+// line streaming wins with the rays per lane: 1.3 M triangles 400,000 rays 317 / 272, 82 k
+// triangles 300,000 / 500,000 / 1 M 113 / 110, 170 / 140, 252 / 199 (in the closed Cornell box,
+// where a ray takes few steps, it costs more than it gains up to 1 M rays: 78 / 79, any hit 49 / 58).
 struct BatchRays
 {
     const SceneView&    s;
@@ -83,12 +94,12 @@ struct BatchRays
     }
 };
 
-template <bool ANY, int MODE, int STACK, int MINB>
+template <bool ANY, int MODE, int STACK, int MINB, bool STREAM>
 __global__ void __launch_bounds__(kTraceBlock, MINB)
     k_trace(SceneView s, const float4* __restrict__ rays, int n, float4* __restrict__ hits, int* __restrict__ occ,
             int* err, unsigned long long* fetch)
 {
-    if constexpr (MODE == 0 && kStreamTraversal)
+    if constexpr (STREAM)
     {
         __shared__ StreamSmem<STACK, kTraceBlock> sm;
         BatchRays q{s, rays, hits, occ, fetch, ANY};
@@ -2918,26 +2929,41 @@ static int trace_impl(mcrt_scene* s, const mcrt_ray* rays, int64_t n, void* out,
     const bool          small = stack_depth(s, traverse) + 2 < kSmallStack;
     // 2^30 rays per launch: the kernels count rays in 32 bits
     constexpr int64_t kSlice = int64_t(1) << 30;
-    auto launch = [&](auto kernel) {
+    auto resident_blocks = [&](auto kernel) {
         int occ = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kTraceBlock, 0);
+        return static_cast<int64_t>(num_sms()) * std::max(occ, 1);
+    };
+    auto launch = [&](auto kernel, int64_t blocks) {
         for (int64_t off = 0; off < n; off += kSlice)
         {
             const int64_t m = std::min(n - off, kSlice);
             if (off > 0) cudaMemsetAsync(d_fetch, 0, sizeof(*d_fetch), st);
             const int64_t want = (m + kTraceBlock - 1) / kTraceBlock;
-            const int     grid =
-                static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(num_sms()) * std::max(occ, 1)));
-            kernel<<<grid, kTraceBlock, 0, st>>>(s->view, d_rays + 2 * off, static_cast<int>(m), any ? nullptr : hits + off,
-                                                 any ? o + off : nullptr, d_err, d_fetch);
+            kernel<<<static_cast<int>(std::min(want, blocks)), kTraceBlock, 0, st>>>(
+                s->view, d_rays + 2 * off, static_cast<int>(m), any ? nullptr : hits + off, any ? o + off : nullptr,
+                d_err, d_fetch);
         }
     };
+    // streamed when some warp gets a second batch (see k_trace)
+    auto launch_fast = [&](auto one_batch, auto streamed) {
+        const int64_t blocks = resident_blocks(one_batch);
+        if (!kStreamTraversal || n <= blocks * kTraceBlock)
+            launch(one_batch, blocks);
+        else
+            launch(streamed, resident_blocks(streamed));
+    };
+    constexpr int  A = kAnyHitMinBlocks, C = kTraceMinBlocks;
+    constexpr bool S = kStreamTraversal;
     if (traverse == MCRT_TRAVERSE_REF)
-        any ? launch(k_trace<true, 1, kStack, 1>) : launch(k_trace<false, 1, kStack, 1>);
+        any ? launch(k_trace<true, 1, kStack, 1, false>, resident_blocks(k_trace<true, 1, kStack, 1, false>))
+            : launch(k_trace<false, 1, kStack, 1, false>, resident_blocks(k_trace<false, 1, kStack, 1, false>));
     else if (small)
-        any ? launch(k_trace<true, 0, kSmallStack, kAnyHitMinBlocks>) : launch(k_trace<false, 0, kSmallStack, kTraceMinBlocks>);
+        any ? launch_fast(k_trace<true, 0, kSmallStack, A, false>, k_trace<true, 0, kSmallStack, A, S>)
+            : launch_fast(k_trace<false, 0, kSmallStack, C, false>, k_trace<false, 0, kSmallStack, C, S>);
     else
-        any ? launch(k_trace<true, 0, kStack, kAnyHitMinBlocks>) : launch(k_trace<false, 0, kStack, kTraceMinBlocks>);
+        any ? launch_fast(k_trace<true, 0, kStack, A, false>, k_trace<true, 0, kStack, A, S>)
+            : launch_fast(k_trace<false, 0, kStack, C, false>, k_trace<false, 0, kStack, C, S>);
     CK(cudaGetLastError());
     int herr = 0;
     if (ptr_mode != MCRT_PTR_DEVICE) CK(cudaMemcpyAsync(out, tmp_out, out_bytes, cudaMemcpyDeviceToHost, st));
