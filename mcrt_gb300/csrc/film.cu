@@ -122,7 +122,8 @@ __global__ void k_film_gamma(float* rgb, int64_t n, float inv_gamma)
 //   k_film_means        a block per channel joins the chunks, 256 at a time; one whose binade or
 //                       end does not fit (about log2 n of them) is redone from s as it is, by the whole
 //                       block, up to each addition that leaves the binade.  The addends of a
-//                       channel that is not covered are added by one thread.
+//                       channel that is not covered, and of an image of one chunk, are added by
+//                       one thread.
 // One thread summing the four channels, a dependent addition and load after another, made the
 // tone mapping of 1023x767 pixels 34.3 ms and of 3840x2160 471 ms; they take 0.23 and 1.4 ms.
 // What is left is latency: about ten passes of one block over the first chunk (a binade each)
@@ -568,9 +569,17 @@ extern "C" int mcrt_film_tonemap(float* rgb, int32_t width, int32_t height, int3
             ChunkInc* d_incs = reinterpret_cast<ChunkInc*>(d_means + 8);
             float*    d_sums = reinterpret_cast<float*>(d_incs + 4 * chunks);
             const int grid = static_cast<int>(chunks);
-            FCK(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
-            k_film_chunk_sums<<<grid, kChunkThreads, 0, st>>>(d_rgb, n, d_sums, d_bad);
-            k_film_chunk_incs<<<grid, kChunkThreads, 0, st>>>(d_rgb, n, d_sums, d_incs, grid);
+            // An image of one chunk: no other chunk's sum to compose it with, and the block's passes over
+            // the chunk (one per binade) take longer than one thread's additions from shared memory.  All
+            // channels go as ones that are not covered (k_film_means), without the two kernels before:
+            // 1 / 527 / 2,048 pixels 63 / 94 / 109 -> 49 / 58 / 64 us a call (2,049 pixels, two chunks: 112).
+            const bool plain = chunks == 1;
+            FCK(cudaMemsetAsync(d_bad, plain ? 0xff : 0, sizeof(int), st));
+            if (!plain)
+            {
+                k_film_chunk_sums<<<grid, kChunkThreads, 0, st>>>(d_rgb, n, d_sums, d_bad);
+                k_film_chunk_incs<<<grid, kChunkThreads, 0, st>>>(d_rgb, n, d_sums, d_incs, grid);
+            }
             k_film_means<<<4, kChunkThreads, 0, st>>>(d_rgb, n, d_incs, grid, d_bad, d_means);
             float means[4];
             FCK(cudaMemcpyAsync(means, d_means, sizeof(means), cudaMemcpyDeviceToHost, st));

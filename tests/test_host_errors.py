@@ -88,7 +88,7 @@ def test_tone_mapping_without_kept_scratch_uses_its_own(cuda):
     """The host thread's kept scratch cannot be allocated: Reinhard takes a smaller buffer of its
     own and the call succeeds (the failed allocation's error is not taken for a launch's)."""
     from mcrt_gb300 import film
-    img = np.ones((5, 7, 3), np.float32)
+    img = np.ones((64, 64, 3), np.float32)
     cuda.fail("cudaMalloc", 2, OUT_OF_MEMORY)  # after the image's device copy
     film.tonemap(img, "reinhard")
     assert cuda.lib.fake_fails_left() == 0
