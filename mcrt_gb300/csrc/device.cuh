@@ -549,7 +549,7 @@ __device__ __forceinline__ bool trace_fast(const SceneView& s, float3 o, float3 
 // What bounds it: instruction issue and the dependent node loads, both made worse by idle
 // lanes -- bounce and next-event rays of one warp take very different numbers of steps, and
 // with one ray per lane and batch 5.9 (next-event) to 9.5 (extension) of 32 lanes were active
-// per instruction.  Here 10-14 are (outdoor frame, 1.3 M triangles: extension rays 47.8 ->
+// per instruction.  Here 13.5 and 15.7 are (outdoor frame, 1.3 M triangles: extension rays 47.8 ->
 // 37.7 ms, next-event rays 33.6 -> 23.3 ms per 67 M paths; 2 M incoherent rays 0.64 -> 0.52 ms).
 //
 //   refill   when kStreamIdle lanes or more are idle: finished rays are handed to q, idle lanes

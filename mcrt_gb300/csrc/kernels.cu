@@ -10,9 +10,9 @@
 //     k_shade            one vertex of rayTrace (demo_pt.cpp:523-651): emission, NEE with
 //                        MIS against the environment and the area lights, continuation,
 //                        Russian roulette, over windows of queue entries sorted by
-//                        material in shared memory; continuing paths, ended paths and
-//                        next-event rays are appended to SoA queues by warp ballot /
-//                        warp prefix sum + one atomic per warp
+//                        material in shared memory; continuing and ended paths are
+//                        appended to SoA queues by ballots and one atomic per block for
+//                        both, next-event rays by one atomic per warp and kind
 //     k_shadow           next-event rays to the environment: any hit
 //     k_connect          next-event rays to area lights: bounded closest hit (which must be
 //                        the sampled emitter), MIS-weighted
@@ -169,24 +169,6 @@ __device__ __forceinline__ unsigned lanemask_lt()
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
-}
-
-// warp-aggregated append: returns this lane's first slot for `k` items
-__device__ __forceinline__ int warp_append(int* counter, int k)
-{
-    const int lane = threadIdx.x & 31;
-    int       incl = k;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1)
-    {
-        int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-    }
-    int total = __shfl_sync(0xffffffffu, incl, 31);
-    int base = 0;
-    if (lane == 31 && total > 0) base = atomicAdd(counter, total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    return base + incl - k;
 }
 
 // adds a path's pending next-event results (bits of `mask` over `slots`) in slot order:
@@ -668,7 +650,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB) k_extend(WaveArgs a, int p)
 // derivative; the vertex's material id goes to the path's log for the other half.
 //
 // What bounds it: the latency of scattered reads (hit normals, materials, environment tables:
-// 9-12 of 19 stall cycles per issue, DRAM 26-34 % busy) and, with an environment, the
+// 9.5 long-scoreboard stall cycles per issue, issue on 36 % of the cycles, DRAM 40 % busy) and, with an environment, the
 // instruction cache.  The continuation is sampled first, so that the path's place in the next
 // queue, and with it the place of its next-event results, is known before the next-event rays
 // are made: each ray is written to its queue as it is made (an array of up to four lay in local
@@ -1530,7 +1512,7 @@ struct Workspace
 };
 
 // One workspace per device, shared by every scene on it.  A render's queues and ring are
-// its largest allocation (about 50 GB at the default 64 M-ray queue); kept per scene, they
+// its largest allocation (about 45 GB at the default 64 M-ray queue); kept per scene, they
 // multiplied by the number of scenes a process holds (the 64-scene mix rendered scene by
 // scene would have kept 412 GB).  A render takes its device's mutex (renders on one device
 // share it anyway); the workspace grows to the largest render and lives until the process
@@ -2751,8 +2733,7 @@ int set_error(int code, const std::string& msg) { return fail(code, msg); }
 namespace {
 struct ThreadScratch
 {
-    void*  ptr = nullptr;
-    size_t bytes = 0;
+    void* ptr = nullptr;
     ~ThreadScratch()
     {
         if (ptr) cudaFree(ptr);  // at thread exit (an error after the runtime is gone is ignored)

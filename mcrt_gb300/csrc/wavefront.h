@@ -53,8 +53,8 @@ constexpr int kAnyHitMinBlocks = 10;
 constexpr int kMaxDepth = 62;
 constexpr int64_t kMaxQueue = int64_t(1) << 27;     // rays per queue (result indices stay in int)
 // Streaming schedule default: 64 M rays (45 GB of queues).  Per cfg1 frame (67 M paths):
-// 1 / 2 / 4 / 8 / 16 / 32 / 64 M rays 184.6 / 146.9 / 128.1 / 118.3 / 113.4 / 111.4 /
-// 109.5 ms -- fewer, longer launches amortise each launch's ramp and tail.  If its
+// 0.5 / 1 / 2 / 4 / 8 / 16 / 32 / 64 M rays 172 / 124 / 99.5 / 86.6 / 81.1 / 78.8 / 77.6 /
+// 78.1 ms -- fewer, longer launches amortise each launch's ramp and tail.  If its
 // allocation fails the default halves itself, down to kMinDefaultQueue.
 constexpr int64_t kDefaultQueue = int64_t(1) << 26;
 constexpr int64_t kMinDefaultQueue = int64_t(1) << 20;
@@ -62,12 +62,12 @@ constexpr int64_t kMinDefaultQueue = int64_t(1) << 20;
 // Counters of one render.  Cleared by: k_extend of parity p lists[p ^ 1], k_shade of parity p
 // the scount and fetch of p ^ 1 (each after their last reader, before their next writer, also
 // with k_shadow / k_connect / k_finish beside the next k_extend).
-// Every warp of k_shade takes places in the ray queue, the finished list and the next-event
-// queues, and waits for the old counts; the L2 answers about one atomic per ns on one line, a
-// million of them per 8 M rays.  So the ray queue and the finished list share one 64-bit counter
-// (one atomic for both), and the counters that are not added to together have lines of their
-// own: Cornell box with a mirror, 8 M rays per launch, k_shade 926 -> 765 and 1100 -> 910 us
-// (first and second vertex).
+// Every block of k_shade takes places in the ray queue and the finished list, every warp in the
+// next-event queues, and waits for the old counts; the L2 answers about one atomic per ns on one
+// line (with an atomic per warp and list, a million of them per 8 M rays).  So the ray queue and
+// the finished list share one 64-bit counter (one atomic for both), and the counters that are not
+// added to together have lines of their own: Cornell box with a mirror, 8 M rays per launch,
+// k_shade 926 -> 765 and 1100 -> 910 us (first and second vertex).
 struct Ctrl
 {
     struct alignas(256) Count
