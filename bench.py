@@ -118,6 +118,14 @@ class ClockSampler:
 K_EXTEND_DRAM_BYTES_PER_RAY = {64: 132.3}
 
 
+def next_event_io_bytes(desc) -> int:
+    """Queue bytes the next-event kernels move per ray, as the least that any ray of this scene needs:
+    an environment ray (k_shadow) reads 32 B and writes nothing unless it is occluded (the counts do
+    not tell occluded rays apart, so the 16 B they clear are left out); an area-light ray (k_connect)
+    reads 64 B of ray, payload and meta and writes its 16-B result."""
+    return 32 if desc.envmap is not None else 64 + 16
+
+
 # rows of the cfg0 / cfg1 frames the CPU port renders for cpu_baseline and --impl reference
 CPU_BASELINE_ROWS = {"cfg0": (64, 192), "cfg1": (384, 640)}
 
@@ -577,10 +585,9 @@ def main():
     # algorithmic bytes of the two traversal kernels: a counting render of the same seeds.
     # k_extend per extension ray: one node fetch per node visited (96 B for the eight-child
     # nodes of the FAST traversal, the sectors a visit touches), 48 B per triangle tested,
-    # 32 B ray + 16 B hit; the next-event kernels per ray: nodes/triangles as above; environment
-    # rays (k_shadow) 32 B in and the 16-B slot an occluded ray clears, area-light rays
-    # (k_connect) 64 B ray + payload + meta in, 16 B result out.  Each launches once per iteration.
-    nee_io = 32 + 16 if args.workload in ("cfg1", "cfg4") else 64 + 16
+    # 32 B ray + 16 B hit; the next-event kernels per ray: nodes/triangles as above and
+    # next_event_io_bytes.  Each launches once per iteration.
+    nee_io = next_event_io_bytes(desc)
     _, sc_cnt = sc.render(cam, seed=0, out=out, profile=PROFILE_COUNT, **kw)
     nb = sc_cnt["node_bytes"]
     # the same counts by bounce class: a depth-0 counting render of the same seeds traces
