@@ -366,10 +366,12 @@ __device__ __forceinline__ void start_camera_path(const WaveArgs& a, int64_t g, 
 // with the arithmetic of FrameBuffer::accumulatePixel / scale.  Called by all 32 lanes.
 //
 // What bounds a frame of few pixels with very many samples: the pixels whose last paths end
-// together are often resolved by one warp, one after another.  Lane c adds channel c from shared
-// memory, 32 samples at a time, while the next 32 are read: 17 ns a sample (three shuffles and
-// adds per sample by all lanes: 42).  Cornell box, 4x3 pixels at 50,000 samples 14.5 -> 9.0 ms,
-// 16x16 at 4,096 5.3 -> 3.2, 64x64 at 1,024 5.4 -> 4.8.
+// together are often resolved by one warp, one after another.  From 32 samples on, lane c adds
+// channel c from shared memory, 32 samples at a time, while the next 32 are read: 17 ns a sample
+// (three shuffles and adds per sample by all lanes: 42).  Cornell box, 4x3 pixels at 50,000
+// samples 14.5 -> 9.0 ms, 16x16 at 4,096 5.3 -> 3.2, 64x64 at 1,024 5.4 -> 4.8.  Fewer samples are
+// shuffled: at one sample a pixel the way through shared memory costs a 61x47 frame 535 us
+// instead of 507.
 //
 // Adjoint (ADJ): the path's radiance L is final here, so each logged Lambert vertex k
 // gets + dL/dI * L / albedo_k; k_shade already added - dL/dI * L_before(k) / albedo_k.
@@ -459,18 +461,20 @@ __device__ __forceinline__ void finish_paths(const WaveArgs& a, const Grads& G, 
             }
             return v;
         };
+        float  s0 = 0.f, s1 = 0.f, s2 = 0.f;
         float4 v = sample(lane);
-        float  sum = 0.f;
-        for (int k0 = 0; k0 < sp; k0 += 32)
+        int    k0 = 0;
+        if (sp >= 32)
         {
-            __syncwarp();
-            rows[0][lane] = v.x;
-            rows[1][lane] = v.y;
-            rows[2][lane] = v.z;
-            __syncwarp();
-            v = sample(k0 + 32 + lane);
-            if (k0 + 32 <= sp)
+            float sum = 0.f;
+            for (; k0 + 32 <= sp; k0 += 32)
             {
+                __syncwarp();
+                rows[0][lane] = v.x;
+                rows[1][lane] = v.y;
+                rows[2][lane] = v.z;
+                __syncwarp();
+                v = sample(k0 + 32 + lane);
 #pragma unroll
                 for (int q = 0; q < 8; ++q)  // sample order
                 {
@@ -481,15 +485,25 @@ __device__ __forceinline__ void finish_paths(const WaveArgs& a, const Grads& G, 
                     sum = sum + f.w;
                 }
             }
-            else
-                for (int l = 0; l < sp - k0; ++l) sum = sum + row[l];
+            s0 = __shfl_sync(0xffffffffu, sum, 0);
+            s1 = __shfl_sync(0xffffffffu, sum, 1);
+            s2 = __shfl_sync(0xffffffffu, sum, 2);
         }
-        if (lane == 0) a.ring_cnt[c0] = 0;
-        if (lane < 3)
+        for (int l = 0; l < sp - k0; ++l)  // the last, fewer than 32
         {
+            s0 += __shfl_sync(0xffffffffu, v.x, l);
+            s1 += __shfl_sync(0xffffffffu, v.y, l);
+            s2 += __shfl_sync(0xffffffffu, v.z, l);
+        }
+        if (lane == 0)
+        {
+            a.ring_cnt[c0] = 0;
             const JobGPU& J = a.jobs[jb];
             const float   scale = static_cast<float>(1.0 / J.spp);  // FrameBuffer::scale(1.0 / spp)
-            J.image[3 * static_cast<int64_t>(px) + lane] = sum * scale;
+            float*        out = J.image + 3 * static_cast<int64_t>(px);
+            out[0] = s0 * scale;
+            out[1] = s1 * scale;
+            out[2] = s2 * scale;
         }
     }
 }
